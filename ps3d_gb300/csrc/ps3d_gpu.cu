@@ -274,11 +274,11 @@ int download(ps3d_gpu_ctx *c, const void *src, bool src_is_fp64, int ncomp, doub
 }
 
 // ------------------------------------------------------------- primitives
-// launches of one line pass over nf fields: one for the FP32 line kernels,
-// one per field otherwise
+// launches of one line pass over nf fields: one for the FP32 and fixed-point
+// line kernels, one per field otherwise
 template <typename T> int line_launches(const ps3d_gpu_ctx *c, int n, int nf)
 {
-    return (sizeof(T) == sizeof(float) && lines32_supported(n)) ? 1 : nf;
+    return (sizeof(T) == sizeof(float) ? lines32_supported(n) : fx_serves(n)) ? 1 : nf;
 }
 // horizontal transforms of nf consecutive fields (nfield apart)
 template <typename T> void xyf(ps3d_gpu_ctx *c, const T *in, T *out, int nf = 1)
@@ -1842,9 +1842,16 @@ void host_tables(ps3d_gpu_ctx *c)
     cudaStreamSynchronize(c->st);  // host vectors go out of scope
 }
 
-template <typename T> void twiddles(ps3d_gpu_ctx *c, void *dst, int n)
+// table of n twiddles; len: the line (or column) length they serve
+template <typename T> void twiddles(ps3d_gpu_ctx *c, void *dst, int n, int len)
 {
     std::vector<CT<T>> tw(n);
+    if (sizeof(T) == sizeof(double) && fx_serves(len)) {
+        fx_twiddles(tw.data(), n);
+        cudaMemcpyAsync(dst, tw.data(), n * sizeof(CT<T>), cudaMemcpyHostToDevice, c->st);
+        cudaStreamSynchronize(c->st);
+        return;
+    }
     for (int k = 0; k < n; ++k) {
         // exact at multiples of pi/2
         double s = sin(2.0 * M_PI * (double)k / (double)n), co = cos(2.0 * M_PI * (double)k / (double)n);
@@ -1957,9 +1964,9 @@ template <typename T> int allocate_fields(ps3d_gpu_ctx *c)
          dalloc(c, &c->flag, sizeof(int)) && dalloc(c, &c->flag_chk, sizeof(int)) && dalloc(c, &c->sc, sizeof(StepScal)) &&
          dalloc(c, &c->roll_dev, c->roll.hist.size() * sizeof(double));
     if (!ok) return fail(c, PS3D_ERR_OUT_OF_MEMORY, "device allocation failed");
-    twiddles<T>(c, c->twx, d.nx);
-    twiddles<T>(c, c->twy, d.ny);
-    twiddles<T>(c, c->twz2, 2 * d.nz);
+    twiddles<T>(c, c->twx, d.nx, d.nx);
+    twiddles<T>(c, c->twy, d.ny, d.ny);
+    twiddles<T>(c, c->twz2, 2 * d.nz, d.nz);
     if (c->fp64) {
         c->twx64 = tf<double2>(c->twx);
         c->twy64 = tf<double2>(c->twy);
@@ -1967,10 +1974,10 @@ template <typename T> int allocate_fields(ps3d_gpu_ctx *c)
         c->phim64 = tf<double>(c->phim);
         c->phip64 = tf<double>(c->phip);
     } else {
-        twiddles<double>(c, c->twx64, d.nx);
-        twiddles<double>(c, c->twy64, d.ny);
-        twiddles<double>(c, c->twz2_64, 2 * d.nz);
-        twiddles<float>(c, c->twz32, d.nz);
+        twiddles<double>(c, c->twx64, d.nx, d.nx);
+        twiddles<double>(c, c->twy64, d.ny, d.ny);
+        twiddles<double>(c, c->twz2_64, 2 * d.nz, d.nz);
+        twiddles<float>(c, c->twz32, d.nz, d.nz);
         std::vector<float> sn(d.nz), cs(d.nz);
         for (int j = 0; j < d.nz; ++j) {
             sn[j] = (float)sin(M_PI * (double)j / (double)d.nz);

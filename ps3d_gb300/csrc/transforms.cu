@@ -108,7 +108,7 @@ int lines_lanes(int n)
 }
 
 // nf fields (field f at in + f fs_in, out + f fs_out): one launch for the
-// FP32 line kernels, one per field otherwise
+// FP32 line kernels and the FP64 ones of fx64.cu, one per field otherwise
 template <typename T>
 void launch_lines(cudaStream_t st, const T *in, T *out, int n, int P, int zv, long long line_stride,
                   long long nbatch, long long batch_stride, bool inverse,
@@ -120,6 +120,13 @@ void launch_lines(cudaStream_t st, const T *in, T *out, int n, int P, int zv, lo
             launch_lines32(st, reinterpret_cast<const float *>(in), reinterpret_cast<float *>(out), n, P, zv,
                            line_stride, nbatch, batch_stride, inverse, reinterpret_cast<const float2 *>(tw), shape,
                            nf, fs_in, fs_out);
+            return;
+        }
+    }
+    if constexpr (sizeof(T) == sizeof(double)) {
+        if (fx_serves(n)) {
+            fx_lines(st, reinterpret_cast<const double *>(in), reinterpret_cast<double *>(out), n, P, zv, line_stride,
+                     nbatch, batch_stride, inverse, tw, nf, fs_in, fs_out);
             return;
         }
     }
@@ -296,6 +303,14 @@ void columns_in(const Dims &d, cudaStream_t st, int mode, const TIN *in, T *out,
                 const T *phip, const typename cplx<T>::type *twz2, Probe *pr)
 {
     if (pr) pr->begin(PROBE_COLUMNS, st);
+    if constexpr (sizeof(T) == sizeof(double) && sizeof(TIN) == sizeof(double)) {
+        if (fx_serves(d.nz)) {
+            fx_columns(d, st, mode, reinterpret_cast<const double *>(in), reinterpret_cast<double *>(out),
+                       reinterpret_cast<const double *>(phim), reinterpret_cast<const double *>(phip), twz2);
+            if (pr) pr->end(PROBE_COLUMNS, st, pass_bytes<T>(d));
+            return;
+        }
+    }
     int B = column_lanes<T>(d.nz);
     const long long ncol = (long long)d.nx * d.ny;
     while (B > 1 && ncol % (2 * B) != 0) B /= 2;
@@ -358,6 +373,7 @@ static void set_smem_attrs()
 void transforms_init()
 {
     lines32_init();
+    fx_init();
     set_smem_attrs<double>();
     set_smem_attrs<float>();
     set_col_attrs<float, double>();
