@@ -12,6 +12,7 @@
 // Everything here is plain integer arithmetic, compiled for host and device:
 // the host build of the same functions is what the CPU test runs.
 #pragma once
+#include <limits.h>
 #include <math.h>
 #include <stdint.h>
 
@@ -41,33 +42,60 @@ FX_FN Half split(long long x)
 {
     Half r;
     r.l = (int)(unsigned)x;
-    r.h = (int)((x >> 32) + (long long)(((unsigned)x) >> 31));
+    r.h = (int)(unsigned)((uint64_t)x >> 32) + (int)(((unsigned)x) >> 31);
     return r;
 }
-FX_FN long long wide(int a, int b) { return (long long)a * (long long)b; }
-
-// round(x w / 2^64) within one unit; |x| < 2^63 - 2^31
-FX_FN long long mulh(Half x, Half w)
+// a b + c, 32 x 32 + 64 bits.  The device form is spelled out: from the C
+// expression the compiler makes separate 64-bit sums (a complex product took
+// 71 instructions, 29 here), and these products at 32 per clock and SM are
+// what the transforms' arithmetic costs most.
+FX_FN long long wide(int a, int b, long long c)
 {
-    const long long mid = wide(x.h, w.l) + wide(x.l, w.h) + 0x80000000ll;
-    return wide(x.h, w.h) + (mid >> 32);
+#ifdef __CUDA_ARCH__
+    long long r;
+    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
+    return r;
+#else
+    return (long long)a * (long long)b + c;
+#endif
 }
-// x c for a constant 0 < c < 1 held as c 2^63 (|x| < 2^62)
-FX_FN long long mulc(long long x, long long c) { return mulh(split(x + x), split(c)); }
+// the upper word, sign extended
+FX_FN long long high(long long m)
+{
+#ifdef __CUDA_ARCH__
+    return (long long)(int)__double2hiint(__longlong_as_double(m));
+#else
+    return m >> 32;
+#endif
+}
+constexpr long long ROUND = 0x80000000ll;
 
-// complex product with a twiddle w = (cos, sin) 2^62 (halves already split):
-// z w / 4
+// c + round(x w / 2^64), the product within one unit; |x| < 2^63 - 2^31
+FX_FN long long mulh(Half x, Half w, long long c = 0)
+{
+    return wide(x.h, w.h, c + high(wide(x.l, w.h, wide(x.h, w.l, ROUND))));
+}
+// x c for a constant 0 < c < 1: c 2^64 where c < 1/2, else x + x (c - 1)
+template <long long CM> FX_FN long long mulc(long long x)
+{
+    constexpr int l = (int)(unsigned)CM, h = (int)((CM >> 32) + (((unsigned)CM) >> 31));
+    return mulh(split(x), Half{h, l}, CM < 0 ? x : 0);
+}
+
+// complex product with a twiddle w = (cos, sin) 2^62 (halves already split,
+// no lower half is -2^31): z w / 4
 struct Tw {
     int ch, cl, sh, sl;
 };
 FX_FN I2 cmulw(I2 z, Tw w, bool conj)
 {
     const Half a = split(z.x), b = split(z.y);
-    const int ph = conj ? -w.sh : w.sh, pl = conj ? -w.sl : w.sl;  // w.y
-    const int nh = conj ? w.sh : -w.sh, nl = conj ? w.sl : -w.sl;  // -w.y
-    const long long mr = wide(a.h, w.cl) + wide(a.l, w.ch) + wide(b.h, nl) + wide(b.l, nh) + 0x80000000ll;
-    const long long mi = wide(b.h, w.cl) + wide(b.l, w.ch) + wide(a.h, pl) + wide(a.l, ph) + 0x80000000ll;
-    return mk2(wide(a.h, w.ch) + wide(b.h, nh) + (mr >> 32), wide(b.h, w.ch) + wide(a.h, ph) + (mi >> 32));
+    const int mh = -w.sh, ml = -w.sl;
+    const int ph = conj ? mh : w.sh, pl = conj ? ml : w.sl;  // w.y
+    const int nh = conj ? w.sh : mh, nl = conj ? w.sl : ml;  // -w.y
+    const long long mr = wide(b.l, nh, wide(b.h, nl, wide(a.l, w.ch, wide(a.h, w.cl, ROUND))));
+    const long long mi = wide(a.l, ph, wide(a.h, pl, wide(b.l, w.ch, wide(b.h, w.cl, ROUND))));
+    return mk2(wide(b.h, nh, wide(a.h, w.ch, high(mr))), wide(a.h, ph, wide(b.h, w.ch, high(mi))));
 }
 // z / 4, rounded
 FX_FN I2 quarter(I2 z) { return mk2((z.x + 2) >> 2, (z.y + 2) >> 2); }
@@ -89,13 +117,13 @@ template <bool INV> FX_FN void dft4(I2 &a0, I2 &a1, I2 &a2, I2 &a3)
     a1 = INV ? mk2(t1.x - u.y, t1.y + u.x) : mk2(t1.x + u.y, t1.y - u.x);
     a3 = INV ? mk2(t1.x + u.y, t1.y - u.x) : mk2(t1.x - u.y, t1.y + u.x);
 }
-constexpr long long C_R2 = 6521908912666391106ll;    // 2^63 / sqrt 2
-constexpr long long C_S3 = 7987674492471257551ll;    // 2^63 sqrt 3 / 2
-constexpr long long C_C1 = 2850178704830799621ll;    // 2^63 cos(2 pi / 5)
-constexpr long long C_C2 = 7461864723258187525ll;    // -2^63 cos(4 pi / 5)
-constexpr long long C_S1 = 8771948077865237882ll;    // 2^63 sin(2 pi / 5)
-constexpr long long C_S2 = 5421362059670026167ll;    // 2^63 sin(4 pi / 5)
-
+// c 2^64, or (c - 1) 2^64 where c >= 1/2
+constexpr long long C_R2 = -5402926248376769404ll;  // 1 / sqrt 2
+constexpr long long C_S3 = -2471395088767036514ll;  // sqrt 3 / 2
+constexpr long long C_C1 = 5700357409661599243ll;  // cos(2 pi / 5)
+constexpr long long C_C2 = -3523014627193176565ll;  // -cos(4 pi / 5)
+constexpr long long C_S1 = -902847917979075853ll;  // sin(2 pi / 5)
+constexpr long long C_S2 = -7604019954369499282ll;  // sin(4 pi / 5)
 template <bool INV> FX_FN void dft8(I2 *v)
 {
     dft4<INV>(v[0], v[2], v[4], v[6]);
@@ -106,8 +134,8 @@ template <bool INV> FX_FN void dft8(I2 *v)
     v[4] = sub(e0, o0);
     if (!INV) {
         // o1 (1 - i)/sqrt2, -i o2, o3 (-1 - i)/sqrt2
-        const long long p = mulc(o1.x + o1.y, C_R2), q = mulc(o1.y - o1.x, C_R2);
-        const long long r = mulc(o3.y - o3.x, C_R2), s = mulc(o3.x + o3.y, C_R2);
+        const long long p = mulc<C_R2>(o1.x + o1.y), q = mulc<C_R2>(o1.y - o1.x);
+        const long long r = mulc<C_R2>(o3.y - o3.x), s = mulc<C_R2>(o3.x + o3.y);
         v[1] = mk2(e1.x + p, e1.y + q);
         v[5] = mk2(e1.x - p, e1.y - q);
         v[2] = mk2(e2.x + o2.y, e2.y - o2.x);
@@ -115,8 +143,8 @@ template <bool INV> FX_FN void dft8(I2 *v)
         v[3] = mk2(e3.x + r, e3.y - s);
         v[7] = mk2(e3.x - r, e3.y + s);
     } else {
-        const long long p = mulc(o1.x - o1.y, C_R2), q = mulc(o1.x + o1.y, C_R2);
-        const long long r = mulc(o3.x + o3.y, C_R2), s = mulc(o3.x - o3.y, C_R2);
+        const long long p = mulc<C_R2>(o1.x - o1.y), q = mulc<C_R2>(o1.x + o1.y);
+        const long long r = mulc<C_R2>(o3.x + o3.y), s = mulc<C_R2>(o3.x - o3.y);
         v[1] = mk2(e1.x + p, e1.y + q);
         v[5] = mk2(e1.x - p, e1.y - q);
         v[2] = mk2(e2.x - o2.y, e2.y + o2.x);
@@ -129,7 +157,7 @@ template <bool INV> FX_FN void dft3(I2 *v)
 {
     const I2 t1 = add(v[1], v[2]), t2 = sub(v[1], v[2]);
     const I2 m = mk2(v[0].x - (t1.x >> 1), v[0].y - (t1.y >> 1));
-    const long long a = mulc(t2.y, C_S3), b = mulc(t2.x, C_S3);
+    const long long a = mulc<C_S3>(t2.y), b = mulc<C_S3>(t2.x);
     const I2 s = INV ? mk2(-a, b) : mk2(a, -b);
     v[0] = add(v[0], t1);
     v[1] = add(m, s);
@@ -138,10 +166,10 @@ template <bool INV> FX_FN void dft3(I2 *v)
 template <bool INV> FX_FN void dft5(I2 *v)
 {
     const I2 t1 = add(v[1], v[4]), t2 = add(v[2], v[3]), t3 = sub(v[1], v[4]), t4 = sub(v[2], v[3]);
-    const I2 m1 = mk2(v[0].x + mulc(t1.x, C_C1) - mulc(t2.x, C_C2), v[0].y + mulc(t1.y, C_C1) - mulc(t2.y, C_C2));
-    const I2 m2 = mk2(v[0].x - mulc(t1.x, C_C2) + mulc(t2.x, C_C1), v[0].y - mulc(t1.y, C_C2) + mulc(t2.y, C_C1));
-    const I2 n1 = mk2(mulc(t3.x, C_S1) + mulc(t4.x, C_S2), mulc(t3.y, C_S1) + mulc(t4.y, C_S2));
-    const I2 n2 = mk2(mulc(t3.x, C_S2) - mulc(t4.x, C_S1), mulc(t3.y, C_S2) - mulc(t4.y, C_S1));
+    const I2 m1 = mk2(v[0].x + mulc<C_C1>(t1.x) - mulc<C_C2>(t2.x), v[0].y + mulc<C_C1>(t1.y) - mulc<C_C2>(t2.y));
+    const I2 m2 = mk2(v[0].x - mulc<C_C2>(t1.x) + mulc<C_C1>(t2.x), v[0].y - mulc<C_C2>(t1.y) + mulc<C_C1>(t2.y));
+    const I2 n1 = mk2(mulc<C_S1>(t3.x) + mulc<C_S2>(t4.x), mulc<C_S1>(t3.y) + mulc<C_S2>(t4.y));
+    const I2 n2 = mk2(mulc<C_S2>(t3.x) - mulc<C_S1>(t4.x), mulc<C_S2>(t3.y) - mulc<C_S1>(t4.y));
     const I2 j1 = INV ? mk2(-n1.y, n1.x) : mk2(n1.y, -n1.x);
     const I2 j2 = INV ? mk2(-n2.y, n2.x) : mk2(n2.y, -n2.x);
     v[0] = add(v[0], add(t1, t2));
@@ -162,18 +190,23 @@ template <int R, bool INV> FX_FN void dft(I2 *v)
 // The passes of a length: radix 8 while 8 divides what is left, one radix 4
 // or 2, then 3s and 5s.  Every pass after the first divides by 4 (its
 // twiddles are held at 2^62 and products keep the upper 64 bits), or by 2
-// (its input is doubled) where the radix is 2, 3 or 4.
+// (its input is doubled) where the radix is below 8.  A line of length
+// 2 odd starts with a 5 or 3 and takes the 2 later.
 FX_FN int next_radix(int rem)
 {
     return rem % 8 == 0 ? 8 : rem % 4 == 0 ? 4 : rem % 2 == 0 ? 2 : rem % 3 == 0 ? 3 : rem % 5 == 0 ? 5 : 1;
 }
-FX_FN constexpr int up_shift(int r) { return r <= 4 ? 1 : 0; }
+FX_FN int first_radix(int n)
+{
+    return n % 8 == 0 ? 8 : n % 4 == 0 ? 4 : n % 5 == 0 ? 5 : n % 3 == 0 ? 3 : 2;
+}
+FX_FN constexpr int up_shift(int r) { return r <= 5 ? 1 : 0; }
 
 // Bits of the fixed-point form.  A line is held in units of 2^(e + 1 - E),
 // 2^e <= its largest magnitude < 2^(e+1): magnitudes up to 2^E.  E is the
 // largest that keeps every modulus of the transform at 2^61.5 or less, which
 // leaves one bit for the sum of two outputs that separates a forward pair
-// and for the doubling inside mulc.  A modulus after the passes of product p
+// and for the doubled input of a small radix.  A modulus after the passes of product p
 // is bounded by p times the largest input and by the sum over the line's
 // inputs: l = ceil(log2(sum / largest)) is measured per line, so that a
 // line with a few large entries (a decaying spectrum) keeps more bits.
@@ -201,7 +234,7 @@ inline Plan make_plan(int n, int mode, int inputs, double scale2)
         down = 0.0;
         passes = 0;
         for (int rem = n; rem > 1; ++passes) {
-            const int r = next_radix(rem);
+            const int r = (mode < 2 && !passes) ? first_radix(n) : next_radix(rem);
             rem /= r;
             lp += log2((double)r);
             if (passes) down += 2.0 - up_shift(r);
@@ -242,7 +275,9 @@ inline void fill_twiddles(Tw *t, int n)
         long double co = swap ? sa : ca, si = swap ? ca : sa;
         if (oct >= 2 && oct < 6) co = -co;
         if (oct >= 4) si = -si;
-        const Half c = split(llrintl(co * one)), s = split(llrintl(-si * one));
+        Half c = split(llrintl(co * one)), s = split(llrintl(-si * one));
+        if (c.l == INT_MIN) c.l += 1;  // its negative has to fit
+        if (s.l == INT_MIN) s.l += 1;
         t[k] = Tw{c.h, c.l, s.h, s.l};
     }
 }
@@ -287,32 +322,40 @@ FX_FN int line_exp(unsigned m)
     const int e = (int)(m >> 20);
     return e < 1 ? 1 : e;
 }
-// x in units of 2^(emax + 1 - E) (emax the unbiased line exponent): the
-// significand at the top of 64 bits, shifted right by 64 - E + (line - own
-// exponent), rounded to nearest (ties away from zero)
+// x in units of 2^(e + 1 - E), e the line's exponent (lexp its biased form):
+// the significand at the top of 64 bits, shifted right by 64 - E and the
+// distance to the line's exponent, the rest dropped.  A subnormal x counts
+// as zero except in lines within 2^-64 of the subnormal range.
 FX_FN long long to_fixed(double x, int lexp, int E)
 {
     const uint64_t u = bits(x);
     const int e = (int)(u >> 52) & 0x7ff;
-    // significand at bits 63..11
-    const uint64_t m = (u << 11) | (e ? 0x8000000000000000ull : 0ull);
-    const int eo = e ? e : 1;
-    const unsigned k = (unsigned)(63 - E + lexp - eo);  // then one more with rounding
-    uint64_t v = k > 63 ? 0 : (m >> k);
-    v = (v + 1) >> 1;
+    uint64_t m = (u << 11) | 0x8000000000000000ull;
+    unsigned k = (unsigned)(63 - E + lexp - e) + 1u;
+    if (lexp < 70 && e == 0) {
+        m = u << 11;
+        k -= 1u;
+    }
+#ifdef __CUDA_ARCH__
+    uint64_t v;
+    asm("shr.u64 %0, %1, %2;" : "=l"(v) : "l"(m), "r"(k));  // amounts above 63 give 0
+#else
+    const uint64_t v = k > 63 ? 0 : m >> k;
+#endif
     const long long s = (long long)u >> 63;
     return ((long long)v ^ s) - s;
 }
-// a magnitude word as FP32, clamped to FP32's normal range
+// a magnitude word as FP32, 0 below FP32's normal range (above it: not a
+// magnitude; spread looks at the line's largest word first)
 FX_FN float magf(unsigned m)
 {
     int t = (int)m - (896 << 20);
-    t = t < 0 ? 0 : t > (254 << 20) ? (254 << 20) : t;
+    t = t < 0 ? 0 : t;
 #ifdef __CUDA_ARCH__
-    return __int_as_float(t << 3);
+    return __int_as_float((int)((unsigned)t << 3));
 #else
     union { float f; int i; } c;
-    c.i = t << 3;
+    c.i = (int)((unsigned)t << 3);
     return c.f;
 #endif
 }
@@ -372,71 +415,83 @@ FX_FN double to_double(long long v, const Scale &s)
 }
 
 // ----- passes
-// One Stockham autosort pass of radix R over nseq groups of B = 2^logB
-// interleaved sequences of length n; element j of lane b at
-// (j << logB) + (b ^ sw(j)) (the XOR keeps accesses along j and along b free
-// of bank conflicts).  Ns: product of the radices already applied.
-// tw[k tws] = exp(-2 pi i k / n) 2^62, halves split.
-FX_FN int sw(int j, int logB)
+// Stockham autosort passes over nseq groups of B = 2^LB interleaved
+// sequences of length n; element j of lane b at (j << LB) + (b ^ sw(j)): the
+// XOR keeps accesses along j and along b free of bank conflicts.
+template <int LB> FX_FN int at(int j, int b)
 {
-    const int B = 1 << logB;
-    return logB >= 3 ? (j & (B - 1)) : ((j >> (3 - logB)) & (B - 1));
+    constexpr int B = 1 << LB;
+    return (j << LB) + (b ^ ((LB >= 3 ? j : j >> (3 - LB)) & (B - 1)));
 }
-FX_FN int at(int j, int b, int logB) { return (j << logB) + (b ^ sw(j, logB)); }
-
-template <int R, bool INV>
-FX_FN void pass(const I2 *src, I2 *dst, int n, int logB, int nseq, int Ns, const Tw *__restrict__ tw, int tws,
-                int tid, int nthreads)
+// One pass of radix R.  Ns: product of the radices already applied;
+// tw[k tws] = exp(-2 pi i k / n) 2^62, halves split.
+template <int R, bool INV, int LB>
+FX_FN void pass(const I2 *src, I2 *dst, int n, int nseq, int Ns, const Tw *__restrict__ tw, int tws, int tid,
+                int nthreads)
 {
-    const int B = 1 << logB;
+    const int B = 1 << LB;
     const int nR = n / R;
-    const int nbf = nR << logB;
-    const int twstride = n / (Ns * R) * tws;
+    const int nbf = nR << LB;
+    const int twstride = nR / Ns * tws;
     for (int g = tid; g < nbf * nseq; g += nthreads) {
-        int s = 0, h = g;
+        int h = g, off = 0;
         while (h >= nbf) {
             h -= nbf;
-            ++s;
+            off += n << LB;
         }
-        const I2 *in = src + (size_t)s * ((size_t)n << logB);
-        I2 *out = dst + (size_t)s * ((size_t)n << logB);
+        const I2 *in = src + off;
+        I2 *out = dst + off;
         const int b = h & (B - 1);
-        const int j = h >> logB;
+        const int j = h >> LB;
         const int k = ((Ns & (Ns - 1)) == 0) ? (j & (Ns - 1)) : (j % Ns);
         I2 v[R];
 #pragma unroll
-        for (int r = 0; r < R; ++r) v[r] = in[at(j + r * nR, b, logB)];
-        if (Ns > 1) {
-            // R = 2, 3, 4 grow by less than 8: doubled first, they divide by 2
-            v[0] = up_shift(R) ? mk2((v[0].x + 1) >> 1, (v[0].y + 1) >> 1) : quarter(v[0]);
+        for (int r = 0; r < R; ++r) v[r] = in[at<LB>(j + r * nR, b)];
+        // a radix below 8: doubled first, so the product divides by 2
+        v[0] = up_shift(R) ? mk2((v[0].x + 1) >> 1, (v[0].y + 1) >> 1) : quarter(v[0]);
+        const Tw *t = tw;
 #pragma unroll
-            for (int r = 1; r < R; ++r) {
-                if (up_shift(R)) v[r] = add(v[r], v[r]);
-                v[r] = cmulw(v[r], tw[k * r * twstride], INV);
-            }
+        for (int r = 1; r < R; ++r) {
+            t += k * twstride;
+            if (up_shift(R)) v[r] = add(v[r], v[r]);
+            v[r] = cmulw(v[r], *t, INV);
         }
         dft<R, INV>(v);
         const int o = (j - k) * R + k;
 #pragma unroll
-        for (int r = 0; r < R; ++r) out[at(o + r * Ns, b, logB)] = v[r];
+        for (int r = 0; r < R; ++r) out[at<LB>(o + r * Ns, b)] = v[r];
     }
 }
-
-// all passes; BAR is the block barrier between passes.  Returns the buffer
-// that holds the result.
-template <bool INV, typename BAR>
-FX_FN I2 *fft(I2 *buf0, I2 *buf1, int n, int logB, int nseq, const Tw *__restrict__ tw, int tws, int tid,
-              int nthreads, BAR bar)
+// the complex spectrum C_k = A_k + i B_k of two packed Hermitian lines from
+// row k and its partner row n - k: A_k = (lo.x, hi.x), B_k = (lo.y, hi.y),
+// lo the row <= n/2
+FX_FN I2 join(I2 own, I2 other, int k, int h)
 {
-    I2 *s = buf0, *d = buf1;
-    int Ns = 1;
-    for (int rem = n; rem > 1;) {
+    if (k == 0 || k == h) return own;
+    return k < h ? mk2(own.x - other.y, other.x + own.y) : mk2(other.x + own.y, other.y - own.x);
+}
+// the first pass (no twiddles): butterfly (j, b) of v, row j + r n / R
+template <int R, bool INV, int LB> FX_FN void first_pass(I2 *v, I2 *dst, int j, int b)
+{
+    dft<R, INV>(v);
+#pragma unroll
+    for (int r = 0; r < R; ++r) dst[at<LB>(j * R + r, b)] = v[r];
+}
+
+// the passes from Ns = ns on (s: buffer that holds the data, d the other);
+// BAR is the block barrier.  Returns the buffer that holds the result.
+template <bool INV, int LB, typename BAR>
+FX_FN I2 *passes(I2 *s, I2 *d, int n, int nseq, int ns, const Tw *__restrict__ tw, int tws, int tid, int nthreads,
+                 BAR bar)
+{
+    int Ns = ns;
+    for (int rem = n / ns; rem > 1;) {
         const int r = next_radix(rem);
-        if (r == 8) pass<8, INV>(s, d, n, logB, nseq, Ns, tw, tws, tid, nthreads);
-        else if (r == 4) pass<4, INV>(s, d, n, logB, nseq, Ns, tw, tws, tid, nthreads);
-        else if (r == 2) pass<2, INV>(s, d, n, logB, nseq, Ns, tw, tws, tid, nthreads);
-        else if (r == 3) pass<3, INV>(s, d, n, logB, nseq, Ns, tw, tws, tid, nthreads);
-        else pass<5, INV>(s, d, n, logB, nseq, Ns, tw, tws, tid, nthreads);
+        if (r == 8) pass<8, INV, LB>(s, d, n, nseq, Ns, tw, tws, tid, nthreads);
+        else if (r == 4) pass<4, INV, LB>(s, d, n, nseq, Ns, tw, tws, tid, nthreads);
+        else if (r == 2) pass<2, INV, LB>(s, d, n, nseq, Ns, tw, tws, tid, nthreads);
+        else if (r == 3) pass<3, INV, LB>(s, d, n, nseq, Ns, tw, tws, tid, nthreads);
+        else pass<5, INV, LB>(s, d, n, nseq, Ns, tw, tws, tid, nthreads);
         bar();
         I2 *t = s;
         s = d;
@@ -445,6 +500,36 @@ FX_FN I2 *fft(I2 *buf0, I2 *buf1, int n, int logB, int nseq, const Tw *__restric
         rem /= r;
     }
     return s;
+}
+// the first pass from shared memory (column sequences)
+template <int R, bool INV, int LB>
+FX_FN void pass1(const I2 *src, I2 *dst, int n, int nseq, int tid, int nthreads)
+{
+    const int nR = n / R, nbf = nR << LB;
+    for (int g = tid; g < nbf * nseq; g += nthreads) {
+        int h = g, off = 0;
+        while (h >= nbf) {
+            h -= nbf;
+            off += n << LB;
+        }
+        const int b = h & ((1 << LB) - 1), j = h >> LB;
+        I2 v[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = src[off + at<LB>(j + r * nR, b)];
+        first_pass<R, INV, LB>(v, dst + off, j, b);
+    }
+}
+template <bool INV, int LB, typename BAR>
+FX_FN I2 *fft(I2 *s, I2 *d, int n, int nseq, const Tw *__restrict__ tw, int tws, int tid, int nthreads, BAR bar)
+{
+    const int r = next_radix(n);
+    if (r == 8) pass1<8, INV, LB>(s, d, n, nseq, tid, nthreads);
+    else if (r == 4) pass1<4, INV, LB>(s, d, n, nseq, tid, nthreads);
+    else if (r == 2) pass1<2, INV, LB>(s, d, n, nseq, tid, nthreads);
+    else if (r == 3) pass1<3, INV, LB>(s, d, n, nseq, tid, nthreads);
+    else pass1<5, INV, LB>(s, d, n, nseq, tid, nthreads);
+    bar();
+    return passes<INV, LB>(d, s, n, nseq, r, tw, tws, tid, nthreads, bar);
 }
 
 // ----- column transforms
@@ -460,17 +545,17 @@ FX_FN I2 *fft(I2 *buf0, I2 *buf1, int n, int logB, int nseq, const Tw *__restric
 // from those at N - j).  No division by sines and no running sums, so no
 // error of a low index reaches the others.  fold forms the inputs of the
 // three FFTs, a quarter each (the factor cmulw brings); W[k] = w^k 2^62.
-// Z at (j << logB) + (p ^ sw(j)); sequence q at seq + q (N << logB).
-template <bool DCT>
-FX_FN void fold(const I2 *Z, I2 *seq, int N, int logB, int p, int j, const Tw *__restrict__ W)
+// Z at (j << LB) + (p ^ sw(j)); sequence q at seq + q (N << LB).
+template <bool DCT, int LB>
+FX_FN void fold(const I2 *Z, I2 *seq, int N, int p, int j, const Tw *__restrict__ W)
 {
     const int n = 2 * N;
-    I2 *s0 = seq, *s1 = seq + ((size_t)N << logB), *s2 = s1 + ((size_t)N << logB);
-    const int q = at(j, p, logB);
+    I2 *s0 = seq, *s1 = seq + ((size_t)N << LB), *s2 = s1 + ((size_t)N << LB);
+    const int q = at<LB>(j, p);
     if (j == 0) {
-        const I2 zN = Z[at(N, p, logB)];
+        const I2 zN = Z[at<LB>(N, p)];
         if (DCT) {
-            const I2 a = Z[q], b = Z[at(n, p, logB)];
+            const I2 a = Z[q], b = Z[at<LB>(n, p)];
             const I2 u = add(a, b), v = add(zN, zN);
             s0[q] = quarter(add(u, v));
             s1[q] = quarter(sub(u, v));
@@ -482,8 +567,8 @@ FX_FN void fold(const I2 *Z, I2 *seq, int N, int logB, int p, int j, const Tw *_
         }
         return;
     }
-    const int qn = at(N - j, p, logB);
-    const I2 a = Z[q], b = Z[at(n - j, p, logB)], c = Z[qn], d = Z[at(N + j, p, logB)];
+    const int qn = at<LB>(N - j, p);
+    const I2 a = Z[q], b = Z[at<LB>(n - j, p)], c = Z[qn], d = Z[at<LB>(N + j, p)];
     const I2 ap = add(a, b), am = sub(a, b), cp = add(c, d), cm = sub(c, d);
     if (DCT) {
         const I2 e0 = quarter(add(ap, cp)), e1 = sub(ap, cp);
@@ -505,13 +590,13 @@ FX_FN void fold(const I2 *Z, I2 *seq, int N, int logB, int p, int j, const Tw *_
 }
 // where Z_m (0 <= m <= n) lies in the transformed sequences: index into the
 // sequences' buffer; *neg where the symmetry changes its sign
-template <bool DCT> FX_FN int unfold(int m, int N, int logB, int p, bool *neg)
+template <bool DCT, int LB> FX_FN int unfold(int m, int N, int p, bool *neg)
 {
     const int r = m & 3;
     *neg = !DCT && r == 3;
     const int k = r == 3 ? (4 * N - m - 1) >> 2 : m >> 2;
     const int s = r == 0 ? 0 : r == 2 ? 1 : 2;
-    return ((s * N) << logB) + at(k, p, logB);
+    return ((s * N) << LB) + at<LB>(k, p);
 }
 
 }  // namespace fx
