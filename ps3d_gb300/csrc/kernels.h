@@ -297,11 +297,18 @@ struct RedOut {
 };
 template <typename T>
 void red_pass1(const Dims &d, cudaStream_t st, const T *vel, const T *vor, double *part, double *result);
+// vortrms from the pass-1 results on the device when res1 is given (FP32
+// form): sqrt(res1[1] / ncell).  The FP64 form screens the strain maxima in
+// est (ncol (nz/32 + 3) floats of scratch) and uses RED2_N + 3 values of result.
 template <typename T>
-// vortrms from the pass-1 results on the device when res1 is given:
-// sqrt(res1[1] / ncell)
 void red_pass2(const Dims &d, cudaStream_t st, const T *vor, const T *g5, double vortrms, double *part,
-               double *result, int *flag, const double *res1 = nullptr, double ncell = 1.0);
+               double *result, int *flag, float *est, const double *res1 = nullptr, double ncell = 1.0);
+template <>
+void red_pass2<float>(const Dims &, cudaStream_t, const float *, const float *, double, double *, double *, int *,
+                      float *, const double *, double);
+template <>
+void red_pass2<double>(const Dims &, cudaStream_t, const double *, const double *, double, double *, double *, int *,
+                       float *, const double *, double);
 int red_nblocks(const Dims &d);
 
 // buoyancy.cu: diffz pieces, flux products, tendency assembly, maximum
@@ -331,7 +338,7 @@ template <typename T>
 void op_bdiag(const Dims &d, cudaStream_t st, const T *b, const T *bx, const T *by, const T *vor, double dzi,
               double bfsq, double *part, double *out);
 constexpr int RED1_N = 12;  // values of pass 1
-constexpr int RED2_N = 5;   // values of pass 2
+constexpr int RED2_N = 5;   // values of pass 2 (the FP64 form's buffer: 3 more)
 
 // tables
 template <typename T>

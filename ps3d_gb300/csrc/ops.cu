@@ -1469,6 +1469,66 @@ __global__ void k_red1(Dims d, const T *__restrict__ vel, const T *__restrict__ 
     block_reduce_store<RED1_N>(vals, kinds, part);
 }
 
+// The FP64 form of pass 1: the sums of a lane's elements of one column are
+// plain fma chains and enter the compensated accumulators once per column,
+// and the maxima compare bit patterns.  The FP64 pipe bounds it: 15
+// operations per element instead of about 50; 256^3: 2174 -> 658 us.
+__device__ __forceinline__ long long order_key(double x)
+{
+    const long long b = __double_as_longlong(x);
+    return b ^ ((b >> 63) & 0x7fffffffffffffffll);  // monotone in x
+}
+__device__ __forceinline__ double key_value(long long k)
+{
+    return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffll));
+}
+template <>
+__global__ void k_red1<double>(Dims d, const double *__restrict__ vel, const double *__restrict__ vor, double *part)
+{
+    const long long N = d.nfield;
+    const long long lowest = order_key(-DBL_MAX);
+    long long vmx[3] = {lowest, lowest, lowest}, wmax2 = 0;
+    Acc<double> s_w2, s_u2, s_h, s_m0, s_m1, s_m2;
+    // NaN: no maximum (as the comparisons of the plain form)
+    const auto raise = [](long long &m, double x) {
+        const long long k = order_key(x);
+        if (k > m && k <= 0x7ff0000000000000ll) m = k;
+    };
+    for (long long col = (long long)blockIdx.x * COLS_PER_BLOCK + threadIdx.y; col < d.ncol;
+         col += (long long)gridDim.x * COLS_PER_BLOCK) {
+        const long long o = col * d.P;
+        double w2c = 0.0, u2c = 0.0, hc = 0.0, m0c = 0.0, m1c = 0.0, m2c = 0.0;
+#pragma unroll 2
+        for (int iz = threadIdx.x; iz <= d.nz; iz += 32) {
+            const long long i = o + iz;
+            const double wt = (iz == 0 || iz == d.nz) ? 0.5 : 1.0;
+            const double x = vor[i], y = vor[N + i], z = vor[2 * N + i];
+            const double u = vel[i], v = vel[N + i], w = vel[2 * N + i];
+            const double w2 = x * x + y * y + z * z;
+            raise(wmax2, w2);
+            w2c += wt * w2;
+            u2c += wt * (u * u + v * v + w * w);
+            hc += wt * (u * x + v * y + w * z);
+            m0c += wt * x;
+            m1c += wt * y;
+            m2c += wt * z;
+            raise(vmx[0], u);
+            raise(vmx[1], v);
+            raise(vmx[2], w);
+        }
+        s_w2.add(w2c);
+        s_u2.add(u2c);
+        s_h.add(hc);
+        s_m0.add(m0c);
+        s_m1.add(m1c);
+        s_m2.add(m2c);
+    }
+    double vals[RED1_N] = {key_value(wmax2), s_w2.value(), s_u2.value(), s_h.value(), s_m0.value(), s_m1.value(),
+                           s_m2.value(), key_value(vmx[0]), key_value(vmx[1]), key_value(vmx[2]), 0.0, 0.0};
+    const int kinds[RED1_N] = {1, 0, 0, 0, 0, 0, 0, 1, 1, 1, 0, 0};
+    block_reduce_store<RED1_N>(vals, kinds, part);
+}
+
 template <typename T>
 void red_pass1(const Dims &d, cudaStream_t st, const T *vel, const T *vor, double *part, double *result)
 {
@@ -1481,50 +1541,44 @@ void red_pass1(const Dims &d, cudaStream_t st, const T *vel, const T *vor, doubl
 
 // Rutishauser cyclic Jacobi eigenvalues of a symmetric 3x3 (jacobi.f90),
 // upper triangle a01 a02 a12, diagonal d0 d1 d2; returns max |lambda|.
-// FP64: the reference's absolute tolerance 1e-15 with a bounded sweep count
-// (*hit set if the bound is reached).  FP32 (unused by the mixed form,
-// which takes the closed form below): the same rotations stopped at FP32
-// resolution after at most 12 sweeps.
-template <typename A>
-__device__ __forceinline__ void givens_rot(A aij, A di, A dj, A &c, A &s, A &t, A &tau)
+// The reference's absolute tolerance 1e-15 with a bounded sweep count (*hit
+// set if the bound is reached).
+__device__ __forceinline__ void givens_rot(double aij, double di, double dj, double &c, double &s, double &t,
+                                           double &tau)
 {
-    const A eps = sizeof(A) == 8 ? (A)DBL_EPSILON : (A)FLT_EPSILON;
-    const A g = (A)100 * fabs(aij);
-    const A h = dj - di;
+    const double eps = DBL_EPSILON;
+    const double g = 100.0 * fabs(aij);
+    const double h = dj - di;
     if (fabs(h) + g == fabs(h)) {
         t = aij / (h + copysign(eps, h));
     } else {
-        const A theta = (A)0.5 * h / (aij + copysign(eps, aij));
-        t = (A)1 / (fabs(theta) + sqrt((A)1 + theta * theta));
-        if (theta < (A)0) t = -t;
+        const double theta = 0.5 * h / (aij + copysign(eps, aij));
+        t = 1.0 / (fabs(theta) + sqrt(1.0 + theta * theta));
+        if (theta < 0.0) t = -t;
     }
-    c = (A)1 / sqrt((A)1 + t * t);
+    c = 1.0 / sqrt(1.0 + t * t);
     s = t * c;
-    tau = s / ((A)1 + c);
+    tau = s / (1.0 + c);
 }
 
-template <typename A>
-__device__ A jacobi_maxabs(A a00, A a01, A a02, A a11, A a12, A a22, int *hit)
+__device__ double jacobi_maxabs(double a00, double a01, double a02, double a11, double a12, double a22, int *hit)
 {
-    A Am[3][3] = {{a00, a01, a02}, {0, a11, a12}, {0, 0, a22}};
-    A D[3] = {a00, a11, a22}, Bv[3] = {a00, a11, a22}, Z[3] = {0, 0, 0};
-    A sm = fabs(Am[0][1]) + fabs(Am[0][2]) + fabs(Am[1][2]);
-    const bool f64 = sizeof(A) == 8;
-    const int maxsweeps = f64 ? 100 : 12;
+    double Am[3][3] = {{a00, a01, a02}, {0, a11, a12}, {0, 0, a22}};
+    double D[3] = {a00, a11, a22}, Bv[3] = {a00, a11, a22}, Z[3] = {0, 0, 0};
+    double sm = fabs(Am[0][1]) + fabs(Am[0][2]) + fabs(Am[1][2]);
     int sweeps = 0;
-    while (f64 ? (sm > (A)1.0e-15)
-               : (sm > (A)1.0e-7 * (fabs(D[0]) + fabs(D[1]) + fabs(D[2])) && sm > (A)1.0e-30)) {
-        if (++sweeps > maxsweeps) {
-            if (f64) *hit = 1;
+    while (sm > 1.0e-15) {
+        if (++sweeps > 100) {
+            *hit = 1;
             break;
         }
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
 #pragma unroll
             for (int j = i + 1; j < 3; ++j) {
-                A c, s, t, tau;
-                givens_rot<A>(Am[i][j], D[i], D[j], c, s, t, tau);
-                A h = t * Am[i][j];
+                double c, s, t, tau;
+                givens_rot(Am[i][j], D[i], D[j], c, s, t, tau);
+                double h = t * Am[i][j];
                 Z[i] -= h;
                 Z[j] += h;
                 D[i] -= h;
@@ -1533,15 +1587,15 @@ __device__ A jacobi_maxabs(A a00, A a01, A a02, A a11, A a12, A a22, int *hit)
 #pragma unroll
                 for (int k = 0; k < 3; ++k) {
                     if (k < i) {
-                        const A g = Am[k][i], hh = Am[k][j];
+                        const double g = Am[k][i], hh = Am[k][j];
                         Am[k][i] = g - s * (hh + g * tau);
                         Am[k][j] = hh + s * (g - hh * tau);
                     } else if (k > i && k < j) {
-                        const A g = Am[i][k], hh = Am[k][j];
+                        const double g = Am[i][k], hh = Am[k][j];
                         Am[i][k] = g - s * (hh + g * tau);
                         Am[k][j] = hh + s * (g - hh * tau);
                     } else if (k > j) {
-                        const A g = Am[i][k], hh = Am[j][k];
+                        const double g = Am[i][k], hh = Am[j][k];
                         Am[i][k] = g - s * (hh + g * tau);
                         Am[j][k] = hh + s * (g - hh * tau);
                     }
@@ -1581,72 +1635,201 @@ __device__ __forceinline__ float sym3_maxabs(float a00, float a01, float a02, fl
     return fmaxf(fabsf(lmax), fabsf(lmin));
 }
 
-template <typename T> struct StrainMax;
-template <> struct StrainMax<double> {
-    __device__ static double get(double a00, double a01, double a02, double a11, double a12, double a22, int *hit)
-    {
-        return jacobi_maxabs<double>(a00, a01, a02, a11, a12, a22, hit);
-    }
-};
-template <> struct StrainMax<float> {
-    __device__ static float get(float a00, float a01, float a02, float a11, float a12, float a22, int *)
-    {
-        return sym3_maxabs(a00, a01, a02, a11, a12, a22);
-    }
-};
-
 // pass 2: 0 vorl1, 1 vorl2 (characteristic vorticity, field_diagnostics.f90:
 // 501-545), 2 ggmax, 3 usggmax, 4 lsggmax (advance.f90:222-276)
-template <typename T>
-__global__ void k_red2(Dims d, const T *__restrict__ vor, const T *__restrict__ g5, double vortrms,
-                       const double *__restrict__ res1, double ncell, double *part, int *flag)
+__global__ void k_red2(Dims d, const float *__restrict__ vor, const float *__restrict__ g5, double vortrms,
+                       const double *__restrict__ res1, double ncell, double *part)
 {
     const long long N = d.nfield;
     // the characteristic-vorticity threshold from the pass-1 results when
     // they stay on the device (sqrt(sum w^2 / ncell), as the host computes)
-    const T vr = (T)(res1 ? sqrt(res1[1] / ncell) : vortrms);
-    Acc<T> l1, l2;
-    T gg = sizeof(T) == 8 ? (T)DBL_EPSILON : (T)FLT_EPSILON, us = 0, ls = 0;
-    int hit = 0;
+    const float vr = (float)(res1 ? sqrt(res1[1] / ncell) : vortrms);
+    Acc<float> l1, l2;
+    float gg = FLT_EPSILON, us = 0, ls = 0;
     for (long long col = (long long)blockIdx.x * COLS_PER_BLOCK + threadIdx.y; col < d.ncol;
          col += (long long)gridDim.x * COLS_PER_BLOCK) {
         const long long o = col * d.P;
         for (int iz = threadIdx.x; iz <= d.nz; iz += 32) {
             const long long i = o + iz;
-            const T x = vor[i], y = vor[N + i], z = vor[2 * N + i];
+            const float x = vor[i], y = vor[N + i], z = vor[2 * N + i];
             if (iz >= 1) {
-                const T v1 = (T)0.5 * fabs(vor[i - 1] + x);
-                const T v2 = (T)0.5 * fabs(vor[N + i - 1] + y);
-                const T v3 = (T)0.5 * fabs(vor[2 * N + i - 1] + z);
+                const float v1 = 0.5f * fabsf(vor[i - 1] + x);
+                const float v2 = 0.5f * fabsf(vor[N + i - 1] + y);
+                const float v3 = 0.5f * fabsf(vor[2 * N + i - 1] + z);
                 if (v1 + v2 + v3 > vr) {
                     l1.add(v1 + v2 + v3);
                     l2.add(v1 * v1 + v2 * v2 + v3 * v3);
                 }
             }
-            const T dudx = g5[i], dudy = g5[N + i], dwdx = g5[2 * N + i], dvdy = g5[3 * N + i],
-                    dwdy = g5[4 * N + i];
-            const T lmax = StrainMax<T>::get(dudx, dudy + (T)0.5 * z, dwdx + (T)0.5 * y, dvdy,
-                                             dwdy - (T)0.5 * x, -(dudx + dvdy), &hit);
-            gg = fmax(gg, lmax);
-            if (iz == d.nz) us = fmax(us, lmax);
-            if (iz == 0) ls = fmax(ls, lmax);
+            const float dudx = g5[i], dudy = g5[N + i], dwdx = g5[2 * N + i], dvdy = g5[3 * N + i],
+                        dwdy = g5[4 * N + i];
+            const float lmax = sym3_maxabs(dudx, dudy + 0.5f * z, dwdx + 0.5f * y, dvdy, dwdy - 0.5f * x,
+                                           -(dudx + dvdy));
+            gg = fmaxf(gg, lmax);
+            if (iz == d.nz) us = fmaxf(us, lmax);
+            if (iz == 0) ls = fmaxf(ls, lmax);
         }
     }
-    if (hit) atomicExch(flag, 1);
     double vals[RED2_N] = {l1.value(), l2.value(), (double)gg, (double)us, (double)ls};
     const int kinds[RED2_N] = {0, 0, 1, 1, 1};
     block_reduce_store<RED2_N>(vals, kinds, part);
 }
 
-template <typename T>
-void red_pass2(const Dims &d, cudaStream_t st, const T *vor, const T *g5, double vortrms, double *part,
-               double *result, int *flag, const double *res1, double ncell)
+// The FP64 form takes the strain maxima from the reference's Jacobi sweeps,
+// but only the points that can hold a maximum need them (256^3: 22.7 ms on the
+// FP64 pipe when every point ran them, 0.71 ms with the screen).  k_red2_screen evaluates the closed form
+// in FP32 at every point and keeps its largest value per chunk of 32 levels;
+// k_strain_max runs the sweeps where the estimate comes within SCREEN of the
+// largest one.  SCREEN is 30 times the estimate's error (the extreme
+// eigenvalues are a few FP32 units off, see sym3_maxabs), so the points that
+// hold the maxima are among them and the results are those of the full sweep.
+// An estimate that is not a number counts as within reach.
+constexpr float SCREEN = 3.0e-5f;
+struct StrainPoint {
+    double a00, a01, a02, a11, a12, a22;
+};
+__device__ __forceinline__ StrainPoint strain_point(const double *__restrict__ vor, const double *__restrict__ g5,
+                                                    long long N, long long i)
 {
-    const int nb = red_grid(d, k_red2<T>);
-    k_red2<T><<<nb, COL_BLOCK, 0, st>>>(d, vor, g5, vortrms, res1, ncell, part, flag);
+    const double dudx = g5[i], dvdy = g5[3 * N + i];
+    return StrainPoint{dudx, g5[N + i] + 0.5 * vor[2 * N + i], g5[2 * N + i] + 0.5 * vor[N + i], dvdy,
+                       g5[4 * N + i] - 0.5 * vor[i], -(dudx + dvdy)};
+}
+__device__ __forceinline__ float strain_estimate(const StrainPoint &s)
+{
+    const float e = sym3_maxabs(narrow32(s.a00), narrow32(s.a01), narrow32(s.a02), narrow32(s.a11), narrow32(s.a12),
+                                narrow32(s.a22));
+    // the closed form's cubes stay inside FP32 between these; all below
+    // count alike, all above as infinite
+    return e < 1.0e-10f ? 1.0e-10f : e > 1.0e12f ? INFINITY : e;
+}
+// est: per column, nz/32 + 1 chunk maxima, then the estimates at iz = nz, 0
+// (infinity where a chunk has an estimate that is not a number)
+__device__ __forceinline__ int est_pitch(int nz) { return (nz >> 5) + 3; }
+__global__ void k_red2_screen(Dims d, const double *__restrict__ vor, const double *__restrict__ g5, double vortrms,
+                              float *__restrict__ est, double *part)
+{
+    const long long N = d.nfield;
+    const double vr2 = 2.0 * vortrms;
+    const int ep = est_pitch(d.nz);
+    Acc<double> l1, l2;
+    float gg = 0.0f, us = 0.0f, ls = 0.0f;
+    for (long long col = (long long)blockIdx.x * COLS_PER_BLOCK + threadIdx.y; col < d.ncol;
+         col += (long long)gridDim.x * COLS_PER_BLOCK) {
+        const long long o = col * d.P;
+        double s1 = 0.0, s2 = 0.0;  // of twice the mid-level magnitudes
+        for (int c0 = 0; c0 <= d.nz; c0 += 32) {
+            const int iz = c0 + threadIdx.x;
+            float e = 0.0f;
+            if (iz <= d.nz) {
+                const long long i = o + iz;
+                if (iz >= 1) {
+                    const double v1 = vor[i - 1] + vor[i], v2 = vor[N + i - 1] + vor[N + i],
+                                 v3 = vor[2 * N + i - 1] + vor[2 * N + i];
+                    const double s = fabs(v1) + fabs(v2) + fabs(v3);
+                    if (s > vr2) {
+                        s1 += s;
+                        s2 += v1 * v1 + v2 * v2 + v3 * v3;
+                    }
+                }
+                e = strain_estimate(strain_point(vor, g5, N, i));
+                gg = fmaxf(gg, e);
+                if (iz == d.nz) {
+                    us = fmaxf(us, e);
+                    est[col * ep + ep - 2] = e;
+                }
+                if (iz == 0) {
+                    ls = fmaxf(ls, e);
+                    est[col * ep + ep - 1] = e;
+                }
+                if (isnan(e)) e = INFINITY;
+            }
+            // non-negative floats order as integers
+            const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(e));
+            if (threadIdx.x == 0) est[col * ep + (c0 >> 5)] = __uint_as_float(m);
+        }
+        l1.add(0.5 * s1);
+        l2.add(0.25 * s2);
+    }
+    double vals[RED2_N] = {l1.value(), l2.value(), (double)gg, (double)us, (double)ls};
+    const int kinds[RED2_N] = {0, 0, 1, 1, 1};
+    block_reduce_store<RED2_N>(vals, kinds, part);
+}
+// top: the largest estimates (k_finish's results 2..4 of the screen); out:
+// the maxima as bit patterns of non-negative doubles, set to their starts
+__global__ void k_strain_max(Dims d, const double *__restrict__ vor, const double *__restrict__ g5,
+                             const float *__restrict__ est, const double *__restrict__ top, unsigned long long *out,
+                             int *flag)
+{
+    const int ep = est_pitch(d.nz), nch = ep - 2;
+    const float lim[3] = {(float)top[0] * (1.0f - SCREEN), (float)top[1] * (1.0f - SCREEN),
+                          (float)top[2] * (1.0f - SCREEN)};
+    const int lane = threadIdx.x & 31;
+    const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
+    // a warp looks at 32 columns' estimates at a time, then takes the chunks
+    // within reach one by one, lanes along z
+    for (long long c0 = warp * 32; c0 < d.ncol; c0 += nw * 32) {
+        for (int ch = 0; ch < nch; ++ch) {
+            bool want = false;
+            if (c0 + lane < d.ncol) {
+                const float *e = est + (c0 + lane) * ep;
+                want = !(e[ch] < lim[0]) || (ch == d.nz >> 5 && !(e[nch] < lim[1])) || (ch == 0 && !(e[nch + 1] < lim[2]));
+            }
+            for (unsigned todo = __ballot_sync(0xffffffffu, want); todo; todo &= todo - 1) {
+                const long long col = c0 + __ffs(todo) - 1;
+                const int iz = ch * 32 + lane;
+                if (iz > d.nz) continue;
+                const StrainPoint s = strain_point(vor, g5, d.nfield, col * d.P + iz);
+                const float e = strain_estimate(s);
+                const bool g = !(e < lim[0]), u = iz == d.nz && !(e < lim[1]), l = iz == 0 && !(e < lim[2]);
+                if (!g && !u && !l) continue;
+                int hit = 0;
+                const double v = jacobi_maxabs(s.a00, s.a01, s.a02, s.a11, s.a12, s.a22, &hit);
+                if (hit) atomicExch(flag, 1);
+                if (isnan(v)) continue;
+                const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+                if (g) atomicMax(out, b);
+                if (u) atomicMax(out + 1, b);
+                if (l) atomicMax(out + 2, b);
+            }
+        }
+    }
+}
+// the screen's largest estimates move behind the results, whose places get
+// the maxima's starts (advance.f90:222: epsilon, 0, 0)
+__global__ void k_strain_start(double *result)
+{
+    for (int k = 0; k < 3; ++k) {
+        result[RED2_N + k] = result[2 + k];
+        result[2 + k] = k ? 0.0 : DBL_EPSILON;
+    }
+}
+
+template <>
+void red_pass2<float>(const Dims &d, cudaStream_t st, const float *vor, const float *g5, double vortrms, double *part,
+                      double *result, int *, float *, const double *res1, double ncell)
+{
+    const int nb = red_grid(d, k_red2);
+    k_red2<<<nb, COL_BLOCK, 0, st>>>(d, vor, g5, vortrms, res1, ncell, part);
     int *kinds;
     cudaGetSymbolAddress((void **)&kinds, c_kinds2);
     k_finish<RED2_N><<<1, dim3(32, RED2_N), 0, st>>>(part, nb, kinds, result);
+}
+template <>
+void red_pass2<double>(const Dims &d, cudaStream_t st, const double *vor, const double *g5, double vortrms,
+                       double *part, double *result, int *flag, float *est, const double *, double)
+{
+    const int nb = red_grid(d, k_red2_screen);
+    k_red2_screen<<<nb, COL_BLOCK, 0, st>>>(d, vor, g5, vortrms, est, part);
+    int *kinds;
+    cudaGetSymbolAddress((void **)&kinds, c_kinds2);
+    k_finish<RED2_N><<<1, dim3(32, RED2_N), 0, st>>>(part, nb, kinds, result);
+    k_strain_start<<<1, 1, 0, st>>>(result);
+    const long long warps = (d.ncol + 31) / 32;
+    const unsigned blocks = (unsigned)((warps + 1) / 2 < 608 ? (warps + 1) / 2 : 608);
+    k_strain_max<<<blocks, 64, 0, st>>>(d, vor, g5, est, result + RED2_N,
+                                        reinterpret_cast<unsigned long long *>(result + 2), flag);
 }
 
 // ------------------------------------------------------------------- tables
@@ -1734,8 +1917,6 @@ void op_hyperbolic_tables(const Dims &d, cudaStream_t st, const double *k2l2, co
     template void op_cn2_update<T>(const Dims &, cudaStream_t, double *, const double *, const T *,           \
                                    const double *, const double *, const double *, double, int);               \
     template void red_pass1<T>(const Dims &, cudaStream_t, const T *, const T *, double *, double *);         \
-    template void red_pass2<T>(const Dims &, cudaStream_t, const T *, const T *, double, double *, double *,  \
-                               int *, const double *, double);                                                 \
     template void op_hyperbolic_tables<T>(const Dims &, cudaStream_t, const double *, const double *,         \
                                           const double *, const double *, const double *, double, T *, T *,   \
                                           T *, T *, T *, T *, T *);

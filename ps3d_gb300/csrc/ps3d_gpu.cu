@@ -818,8 +818,11 @@ template <typename T> int adapt(ps3d_gpu_ctx *c, double t, double *dt_out, ps3d_
     c->launches += 1;
     xyi<T>(c, g5, g5, 5);
     cudaMemsetAsync(c->flag, 0, sizeof(int), c->st);
-    red_pass2<T>(d, c->st, tf<T>(c->vor), g5, vortrms, c->part, c->res2, c->flag);
-    c->launches += 2;
+    // tmp field 5 is free here (the gradients fill 0..4): the FP64 form's
+    // strain estimates, (nz/32 + 3) floats per column
+    red_pass2<T>(d, c->st, tf<T>(c->vor), g5, vortrms, c->part, c->res2, c->flag,
+                 reinterpret_cast<float *>(tmpf<T>(c, 5)));
+    c->launches += c->fp64 ? 4 : 2;
     double r2[RED2_N];
     int hflag = 0;
     cudaMemcpyAsync(r2, c->res2, RED2_N * sizeof(double), cudaMemcpyDeviceToHost, c->st);
@@ -1247,7 +1250,8 @@ int dev_pre(ps3d_gpu_ctx *c)
     c->launches += 3;
     for (int k = 0; k < 5; ++k) xyi<float>(c, g5 + k * N, g5 + k * N);
     cudaMemsetAsync(c->flag, 0, sizeof(int), c->st);
-    red_pass2<float>(d, c->st, tf<float>(c->vor), g5, 0.0, c->part, c->res2, c->flag, c->res1, (double)c->ncell);
+    red_pass2<float>(d, c->st, tf<float>(c->vor), g5, 0.0, c->part, c->res2, c->flag, nullptr, c->res1,
+                     (double)c->ncell);
     c->launches += 2;
     AdaptParams ap;
     ap.cflmax = c->cfg.cflmax;
@@ -1960,7 +1964,7 @@ template <typename T> int allocate_fields(ps3d_gpu_ctx *c)
          dalloc(c, &c->zm, Z) && dalloc(c, &c->zp, Z) && dalloc(c, &c->ubar, Z) && dalloc(c, &c->vbar, Z) &&
          dalloc(c, &c->ini, 2 * sizeof(double)) && dalloc(c, &c->savg, 2 * sizeof(double)) &&
          dalloc(c, &c->part, (size_t)red_nblocks(d) * RED1_N * sizeof(double)) &&
-         dalloc(c, &c->res1, RED1_N * sizeof(double)) && dalloc(c, &c->res2, RED2_N * sizeof(double)) &&
+         dalloc(c, &c->res1, RED1_N * sizeof(double)) && dalloc(c, &c->res2, (RED2_N + 3) * sizeof(double)) &&
          dalloc(c, &c->flag, sizeof(int)) && dalloc(c, &c->flag_chk, sizeof(int)) && dalloc(c, &c->sc, sizeof(StepScal)) &&
          dalloc(c, &c->roll_dev, c->roll.hist.size() * sizeof(double));
     if (!ok) return fail(c, PS3D_ERR_OUT_OF_MEMORY, "device allocation failed");
