@@ -189,7 +189,7 @@ void fx_lines(cudaStream_t st, const double *in, double *out, int n, int P, int 
 // (fx.cuh), transformed together and unfolded by the same warps.
 template <int MODE, int LB>
 __global__ void __launch_bounds__(256) k_fx_columns(const double *__restrict__ in, double *__restrict__ out, int nz,
-                                                    int P, long long ncol, const double *__restrict__ phim,
+                                                    int P, long long ncol, long long fs, const double *__restrict__ phim,
                                                     const double *__restrict__ phip, const __grid_constant__ fx::Plan pl,
                                                     const Tw *__restrict__ W)
 {
@@ -206,6 +206,8 @@ __global__ void __launch_bounds__(256) k_fx_columns(const double *__restrict__ i
     double *raw = reinterpret_cast<double *>(Z);
     const long long col0 = (long long)blockIdx.x * 2 * B;
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
+    in += blockIdx.y * fs;
+    out += blockIdx.y * fs;
 
     for (int cl = warp; cl < 2 * B; cl += nt >> 5) {
         const int p = cl >> 1, comp = cl & 1;
@@ -270,17 +272,17 @@ __global__ void __launch_bounds__(256) k_fx_columns(const double *__restrict__ i
 
 template <int MODE, int LB>
 static void launch_fx_columns(const Dims &d, cudaStream_t st, const double *in, double *out, const double *phim,
-                              const double *phip, const Tw *W)
+                              const double *phip, const Tw *W, int nf)
 {
-    const unsigned grid = (unsigned)((d.ncol + (2 << LB) - 1) / (2 << LB));
-    k_fx_columns<MODE, LB><<<grid, 256, (size_t)d.nz * 48 << LB, st>>>(in, out, d.nz, d.P, d.ncol, phim, phip,
-                                                                       fx::col_plan(d.nz), W);
+    const dim3 grid((unsigned)((d.ncol + (2 << LB) - 1) / (2 << LB)), (unsigned)nf);
+    k_fx_columns<MODE, LB><<<grid, 256, (size_t)d.nz * 48 << LB, st>>>(in, out, d.nz, d.P, d.ncol, d.nfield, phim,
+                                                                       phip, fx::col_plan(d.nz), W);
 }
 
 void fx_columns(const Dims &d, cudaStream_t st, int mode, const double *in, double *out, const double *phim,
-                const double *phip, const void *tw)
+                const double *phip, const void *tw, int nf)
 {
-    auto go = [&](auto f) { f(d, st, in, out, phim, phip, reinterpret_cast<const Tw *>(tw)); };
+    auto go = [&](auto f) { f(d, st, in, out, phim, phip, reinterpret_cast<const Tw *>(tw), nf); };
     // pairs per block: 8, or 4 where the buffers would pass 64 KiB
     const bool wide = d.nz * 48 * 8 <= 64 * 1024;
     switch (mode) {

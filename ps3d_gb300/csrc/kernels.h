@@ -75,7 +75,7 @@ void xy_inverse(const Dims &d, cudaStream_t st, const T *in, T *out, const typen
                 const typename cplx<T>::type *twy, Probe *pr, int nf = 1);
 template <typename T>
 void columns(const Dims &d, cudaStream_t st, int mode, const T *in, T *out, const T *phim,
-             const T *phip, const typename cplx<T>::type *twz2, Probe *pr);
+             const T *phip, const typename cplx<T>::type *twz2, Probe *pr, int nf = 1);
 // FP64 transforms on the integer pipes (fx64.cu).  Lengths up to 512: there
 // the fixed-point error is below an FP64 FFT's on every kind of line
 // measured; at 1024 a decaying spectrum would lose (5e-16 against 2e-16).
@@ -87,8 +87,9 @@ void fx_init();
 void fx_lines(cudaStream_t st, const double *in, double *out, int n, int P, int zv, long long line_stride,
               long long nbatch, long long batch_stride, bool inverse, const void *tw, int nf, long long fs_in,
               long long fs_out);
+// nf consecutive fields (nfield apart) in one launch
 void fx_columns(const Dims &d, cudaStream_t st, int mode, const double *in, double *out, const double *phim,
-                const double *phip, const void *tw);
+                const double *phip, const void *tw, int nf);
 // FP32 bandwidth-tuned line FFTs (lines32.cu), n = 64..1024
 bool lines32_supported(int n);
 void lines32_init();

@@ -380,6 +380,8 @@ void op_products_dz(const Dims &d, cudaStream_t st, double dzi, const T *vel, co
 {
     k_products_dz<T><<<col_grid(d), COL_BLOCK, 0, st>>>(d, (T)dzi, (T)(0.5 * dzi), vel, vor, r, q, p, gq, gp);
 }
+template void op_products_dz<double>(const Dims &, cudaStream_t, double, const double *, const double *, double *,
+                                     double *, double *, double *, double *);
 template void op_products_dz<float>(const Dims &, cudaStream_t, double, const float *, const float *, float *,
                                     float *, float *, float *, float *);
 

@@ -310,6 +310,14 @@ template <typename T, typename TIN> void col_any(ps3d_gpu_ctx *c, int mode, cons
     c->launches += NL_COL;
 }
 template <typename T> void col(ps3d_gpu_ctx *c, int mode, const T *in, T *out) { col_any<T, T>(c, mode, in, out); }
+// nf consecutive FP64 columns fields (nfield apart), one launch where the
+// fixed-point kernel serves the length
+void col64(ps3d_gpu_ctx *c, int mode, const double *in, double *out, int nf)
+{
+    columns<double>(c->d, c->st, mode, in, out, tf<double>(c->phim), tf<double>(c->phip), tf<double2>(c->twz2),
+                    &c->probe, nf);
+    c->launches += fx_serves(c->d.nz) ? 1 : nf;
+}
 // a T view of an FP64 state component (copy for the mixed form)
 template <typename T> const T *state_as_T(ps3d_gpu_ctx *c, const double *s, T *scratch)
 {
@@ -379,11 +387,9 @@ void project_state_mixed(ps3d_gpu_ctx *c)
 // linear and commutes with the per-column integrating factors, so the
 // projected trajectory is the reference's), which keeps FP32 rounding out of
 // the prognostic state; vor2vel then only evaluates vor, vel and svel.
-template <typename T> int vor2vel_mixed(ps3d_gpu_ctx *c);
-
-template <typename T> int vor2vel(ps3d_gpu_ctx *c)
+int vor2vel_fp64(ps3d_gpu_ctx *c)
 {
-    if (sizeof(T) == sizeof(float)) return vor2vel_mixed<T>(c);
+    using T = double;
     const Dims &d = c->d;
     const long long N = d.nfield;
     double *A = c->svor, *B = c->svor + N, *Cc = c->svor + 2 * N;
@@ -394,18 +400,20 @@ template <typename T> int vor2vel(ps3d_gpu_ctx *c)
 
     // solenoidal projection (inversion.f90:34-76)
     op_v2v_ds<T, double>(d, c->st, D, A, B, ds);
-    col<T>(c, COL_COMBINE, state_as_T<T>(c, Cc, bs), cs);
+    col<T>(c, COL_COMBINE, Cc, cs);
     op_diffz<T>(d, c->st, c->dzi, cs, es);
     col<T>(c, COL_DECOMP, es, es);
     op_v2v_project<T, double>(d, c->st, D, c->k2l2i, es, ds, A, B);
     c->launches += 3;
 
-    // vorticity in physical space (field_combine_physical x3, :80-82)
-    col<T>(c, COL_COMBINE, state_as_T<T>(c, A, bs), bs);
-    xyi<T>(c, bs, vor);
-    col<T>(c, COL_COMBINE, state_as_T<T>(c, B, bs), bs);
-    xyi<T>(c, bs, vor + N);
-    xyi<T>(c, cs, vor + 2 * N);
+    // vorticity in physical space (field_combine_physical x3, :80-82): the
+    // first two components combined straight into vor, x lines of those in
+    // place and of cs into the third, then the y lines of all three
+    col64(c, COL_COMBINE, A, vor, 2);
+    x_inverse<T>(d, c->st, vor, vor, tf<CT<T>>(c->twx), &c->probe, 2);
+    x_inverse<T>(d, c->st, cs, vor + 2 * N, tf<CT<T>>(c->twx), &c->probe, 1);
+    y_inverse<T>(d, c->st, vor, vor, tf<CT<T>>(c->twy), &c->probe, 3);
+    c->launches += line_launches<T>(c, d.nx, 2) + line_launches<T>(c, d.nx, 1) + line_launches<T>(c, d.ny, 3);
 
     // vertical velocity (:86-139)
     op_v2v_wsrc<T, double>(d, c->st, D, A, B, ds);
@@ -418,7 +426,7 @@ template <typename T> int vor2vel(ps3d_gpu_ctx *c)
     op_v2v_meanflow<double>(d, c->st, A, B, c->tables(), c->ubar, c->vbar);
     op_v2v_uv<T>(d, c->st, D, c->k2l2i, es, cs, c->ubar, c->vbar, svel, svel + N);
     c->launches += 5;
-    for (int k = 0; k < 3; ++k) xyi<T>(c, svel + k * N, vel + k * N);
+    xyi<T>(c, svel, vel, 3);
     return check(c, "vor2vel");
 }
 
@@ -478,6 +486,12 @@ template <typename T> int vor2vel_mixed(ps3d_gpu_ctx *c)
     c->launches += 2;
     xyi<T>(c, svel, vel, 3);
     return check(c, "vor2vel");
+}
+
+template <typename T> int vor2vel(ps3d_gpu_ctx *c)
+{
+    if constexpr (sizeof(T) == sizeof(float)) return vor2vel_mixed<T>(c);
+    else return vor2vel_fp64(c);
 }
 
 // The tail of the mixed source: the three tendency components decomposed
@@ -689,16 +703,9 @@ template <typename T> int source(ps3d_gpu_ctx *c)
         x_forward<float>(d, c->st, reinterpret_cast<const float *>(r), reinterpret_cast<float *>(r),
                          tf<float2>(c->twx), &c->probe, 5);
         c->launches += line_launches<float>(c, d.nx, 5);
-    } else if (sizeof(T) == sizeof(float)) {
-        op_products_dz<float>(d, c->st, c->dzi, reinterpret_cast<const float *>(vel),
-                              reinterpret_cast<const float *>(vor), tf<float>(r), tf<float>(q), tf<float>(p),
-                              tf<float>(gq), tf<float>(gp));
-        c->launches += 1;
     } else {
-        op_products<T>(d, c->st, vel, vor, r, q, p);
-        op_diffz<T>(d, c->st, c->dzi, q, gq);
-        op_diffz<T>(d, c->st, c->dzi, p, gp);
-        c->launches += 3;
+        op_products_dz<T>(d, c->st, c->dzi, vel, vor, r, q, p, gq, gp);
+        c->launches += 1;
     }
     if (c->cfg.buoyancy) {
         op_addf<T>(d, c->st, r, tf<T>(c->buoy));  // c->buoy from buoyancy_tendency
@@ -734,12 +741,12 @@ template <typename T> int source(ps3d_gpu_ctx *c)
         source_decompose_mixed<T>(c);
         return check(c, "source");
     }
-    for (int k = 0; k < 5; ++k) {
-        xyf<T>(c, f5[k], f5[k]);
-        col<T>(c, COL_DECOMP, f5[k], f5[k]);
-    }
+    // FP64: as above, assembled before the decomposition (the five products
+    // are consecutive); the closure's correction comes decomposed
+    xyf<T>(c, r, r, 5);
     op_svorts<T>(d, c->st, c->D(), r, q, p, gq, gp, svorts, svorts + N, svorts + 2 * N);
     c->launches += 1;
+    if constexpr (sizeof(T) == sizeof(double)) col64(c, COL_DECOMP, svorts, svorts, 3);
     if (c->closure) closure_add<T>(c, svorts);
     return check(c, "source");
 }

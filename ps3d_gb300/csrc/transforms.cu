@@ -303,14 +303,6 @@ void columns_in(const Dims &d, cudaStream_t st, int mode, const TIN *in, T *out,
                 const T *phip, const typename cplx<T>::type *twz2, Probe *pr)
 {
     if (pr) pr->begin(PROBE_COLUMNS, st);
-    if constexpr (sizeof(T) == sizeof(double) && sizeof(TIN) == sizeof(double)) {
-        if (fx_serves(d.nz)) {
-            fx_columns(d, st, mode, reinterpret_cast<const double *>(in), reinterpret_cast<double *>(out),
-                       reinterpret_cast<const double *>(phim), reinterpret_cast<const double *>(phip), twz2);
-            if (pr) pr->end(PROBE_COLUMNS, st, pass_bytes<T>(d));
-            return;
-        }
-    }
     int B = column_lanes<T>(d.nz);
     const long long ncol = (long long)d.nx * d.ny;
     while (B > 1 && ncol % (2 * B) != 0) B /= 2;
@@ -336,9 +328,18 @@ void columns_in(const Dims &d, cudaStream_t st, int mode, const TIN *in, T *out,
 
 template <typename T>
 void columns(const Dims &d, cudaStream_t st, int mode, const T *in, T *out, const T *phim,
-             const T *phip, const typename cplx<T>::type *twz2, Probe *pr)
+             const T *phip, const typename cplx<T>::type *twz2, Probe *pr, int nf)
 {
-    columns_in<T, T>(d, st, mode, in, out, phim, phip, twz2, pr);
+    if constexpr (sizeof(T) == sizeof(double)) {
+        if (fx_serves(d.nz)) {
+            if (pr) pr->begin(PROBE_COLUMNS, st);
+            fx_columns(d, st, mode, in, out, phim, phip, twz2, nf);
+            if (pr) pr->end(PROBE_COLUMNS, st, nf * pass_bytes<T>(d));
+            return;
+        }
+    }
+    for (int f = 0; f < nf; ++f)
+        columns_in<T, T>(d, st, mode, in + f * d.nfield, out + f * d.nfield, phim, phip, twz2, pr);
 }
 
 size_t lines_smem_bytes(int n, bool fp64)
@@ -387,13 +388,15 @@ template void xy_inverse<double>(const Dims &, cudaStream_t, const double *, dou
                                  const double2 *, Probe *, int);
 template void xy_inverse<float>(const Dims &, cudaStream_t, const float *, float *, const float2 *,
                                 const float2 *, Probe *, int);
+template void x_inverse<double>(const Dims &, cudaStream_t, const double *, double *, const double2 *, Probe *, int);
+template void y_inverse<double>(const Dims &, cudaStream_t, const double *, double *, const double2 *, Probe *, int);
 template void x_forward<float>(const Dims &, cudaStream_t, const float *, float *, const float2 *, Probe *, int);
 template void x_inverse<float>(const Dims &, cudaStream_t, const float *, float *, const float2 *, Probe *, int);
 template void y_inverse<float>(const Dims &, cudaStream_t, const float *, float *, const float2 *, Probe *, int);
 template void columns<double>(const Dims &, cudaStream_t, int, const double *, double *, const double *,
-                              const double *, const double2 *, Probe *);
+                              const double *, const double2 *, Probe *, int);
 template void columns<float>(const Dims &, cudaStream_t, int, const float *, float *, const float *,
-                             const float *, const float2 *, Probe *);
+                             const float *, const float2 *, Probe *, int);
 template void columns_in<float, double>(const Dims &, cudaStream_t, int, const double *, float *, const float *,
                                        const float *, const float2 *, Probe *);
 
