@@ -1,4 +1,4 @@
-// FP64 line and column transforms on the integer pipes (fx.cuh).
+// FP64 line transforms on the integer pipes (fx.cuh).
 //
 // Measured per field, one launch.  128^3: line passes 81-90 us with the FP64
 // Stockham kernels, which the FP64 pipe bounds, 33-36 us in the first
@@ -28,7 +28,7 @@ using fx::Tw;
 // passes go through shared memory, 16 bytes per complex value each way.
 template <int R1, bool INV, int LB>
 __global__ void __launch_bounds__(R1 == 8 ? 256 : 512)
-    k_fx_lines(const double *__restrict__ in, double *__restrict__ out, int n, int P, int zv, long long line_stride,
+    k_fx_lines(const double *in, double *out, int n, int P, int zv, long long line_stride,
                long long batch_stride, long long fs_in, long long fs_out, const __grid_constant__ fx::Plan pl,
                const Tw *__restrict__ tw)
 {
@@ -178,121 +178,6 @@ void fx_lines(cudaStream_t st, const double *in, double *out, int n, int P, int 
     else go(launch_fx_lines<3, 1>);
 }
 
-// ------------------------------------------------------------------------
-// z column transforms (dst / dct of src/fft/stafft.f90:410-550), with the
-// harmonic parts of field_decompose_semi_spectral / field_combine_semi_spectral
-// (inversion_utils.f90:563-647) in FP64 as in k_columns (transforms.cu)
-// ------------------------------------------------------------------------
-// A block owns 2B columns (B packed pairs).  A warp takes one column at a
-// time (lanes along z: coalesced) and finds that column's scale by shuffles
-// alone; the pairs are then folded into the three half-length sequences
-// (fx.cuh), transformed together and unfolded by the same warps.
-template <int MODE, int LB>
-__global__ void __launch_bounds__(256) k_fx_columns(const double *__restrict__ in, double *__restrict__ out, int nz,
-                                                    int P, long long ncol, long long fs, const double *__restrict__ phim,
-                                                    const double *__restrict__ phip, const __grid_constant__ fx::Plan pl,
-                                                    const Tw *__restrict__ W)
-{
-    constexpr bool DCT = MODE == COL_DCT;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ double bnd[16][2];
-    __shared__ unsigned smag[16];
-    __shared__ int sbits[16];
-    constexpr int B = 1 << LB;
-    const int N = nz / 2;
-    I2 *seq = reinterpret_cast<I2 *>(smem_raw);
-    I2 *Z = seq + ((3 * N) << LB);  // 3N >= nz + 1
-    long long *Zs = reinterpret_cast<long long *>(Z);
-    double *raw = reinterpret_cast<double *>(Z);
-    const long long col0 = (long long)blockIdx.x * 2 * B;
-    const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
-    in += blockIdx.y * fs;
-    out += blockIdx.y * fs;
-
-    for (int cl = warp; cl < 2 * B; cl += nt >> 5) {
-        const int p = cl >> 1, comp = cl & 1;
-        const long long o = (col0 + cl) * P;
-        const bool on = col0 + cl < ncol;
-        const double f0 = on ? in[o] : 0.0, fn = on ? in[o + nz] : 0.0;
-        unsigned m = 0u;
-        float t = 0.0f;
-        for (int iz = lane; iz <= nz; iz += 32) {
-            double v = 0.0;
-            if (on && (DCT || (iz > 0 && iz < nz))) {
-                v = in[o + iz];
-                if (MODE == COL_DECOMP) v = v - (f0 * phim[o + iz] + fn * phip[o + iz]);
-            }
-            raw[2 * fx::at<LB>(iz, p) + comp] = v;
-            const unsigned a = fx::mag(v);
-            m = max(m, a);
-            t += fx::magf(a);
-        }
-        m = __reduce_max_sync(0xffffffffu, m);
-        for (int q = 16; q > 0; q >>= 1) t += __shfl_xor_sync(0xffffffffu, t, q);
-        const int E = pl.E[fx::spread(t, m, pl.lcap)], e = fx::line_exp(m);
-        for (int iz = lane; iz <= nz; iz += 32) {
-            const int q = 2 * fx::at<LB>(iz, p) + comp;
-            Zs[q] = fx::to_fixed(raw[q], e, E);
-        }
-        if (lane == 0) {
-            bnd[cl][0] = f0;
-            bnd[cl][1] = fn;
-            smag[cl] = m;
-            sbits[cl] = E;
-        }
-    }
-    __syncthreads();
-    for (int g = tid; g < (N / 2 + 1) << LB; g += nt) fx::fold<DCT, LB>(Z, seq, N, g & (B - 1), g >> LB, W);
-    __syncthreads();
-    const I2 *res = fx::fft<false, LB>(seq, Z, N, 3, W, 4, tid, nt, [] { __syncthreads(); });
-    const long long *rs = reinterpret_cast<const long long *>(res);
-    for (int cl = warp; cl < 2 * B; cl += nt >> 5) {
-        if (col0 + cl >= ncol) return;
-        const int p = cl >> 1, comp = cl & 1;
-        const long long o = (col0 + cl) * P;
-        const double f0 = bnd[cl][0], fn = bnd[cl][1];
-        const fx::Scale s = fx::scale_of(smag[cl], sbits[cl], pl);
-        for (int iz = lane; iz <= nz; iz += 32) {
-            bool neg;
-            const int q = fx::unfold<DCT, LB>(iz, N, p, &neg);
-            // the dst is -Im Z of the first column and, i times it being
-            // the packed second one, Re Z
-            long long x = rs[2 * q + (DCT ? comp : 1 - comp)];
-            if (!DCT && (comp == 0) != neg) x = -x;
-            double v = fx::to_double(x, s);
-            if (MODE == COL_COMBINE) v = v + f0 * phim[o + iz] + fn * phip[o + iz];
-            if (!DCT) {
-                if (iz == 0) v = f0;
-                if (iz == nz) v = MODE == COL_DST ? 0.0 : fn;
-            }
-            out[o + iz] = v;
-        }
-    }
-}
-
-template <int MODE, int LB>
-static void launch_fx_columns(const Dims &d, cudaStream_t st, const double *in, double *out, const double *phim,
-                              const double *phip, const Tw *W, int nf)
-{
-    const dim3 grid((unsigned)((d.ncol + (2 << LB) - 1) / (2 << LB)), (unsigned)nf);
-    k_fx_columns<MODE, LB><<<grid, 256, (size_t)d.nz * 48 << LB, st>>>(in, out, d.nz, d.P, d.ncol, d.nfield, phim,
-                                                                       phip, fx::col_plan(d.nz), W);
-}
-
-void fx_columns(const Dims &d, cudaStream_t st, int mode, const double *in, double *out, const double *phim,
-                const double *phip, const void *tw, int nf)
-{
-    auto go = [&](auto f) { f(d, st, in, out, phim, phip, reinterpret_cast<const Tw *>(tw), nf); };
-    // pairs per block: 8, or 4 where the buffers would pass 64 KiB
-    const bool wide = d.nz * 48 * 8 <= 64 * 1024;
-    switch (mode) {
-    case COL_DST: wide ? go(launch_fx_columns<COL_DST, 3>) : go(launch_fx_columns<COL_DST, 2>); break;
-    case COL_DCT: wide ? go(launch_fx_columns<COL_DCT, 3>) : go(launch_fx_columns<COL_DCT, 2>); break;
-    case COL_DECOMP: wide ? go(launch_fx_columns<COL_DECOMP, 3>) : go(launch_fx_columns<COL_DECOMP, 2>); break;
-    default: wide ? go(launch_fx_columns<COL_COMBINE, 3>) : go(launch_fx_columns<COL_COMBINE, 2>); break;
-    }
-}
-
 bool fx_serves(int n) { return n <= 512; }
 void fx_twiddles(void *host, int n) { fx::fill_twiddles(reinterpret_cast<Tw *>(host), n); }
 
@@ -300,11 +185,6 @@ template <int R1, int LB> static void fx_line_attrs()
 {
     cudaFuncSetAttribute(k_fx_lines<R1, true, LB>, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024);
     cudaFuncSetAttribute(k_fx_lines<R1, false, LB>, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024);
-}
-template <int MODE> static void fx_col_attrs()
-{
-    cudaFuncSetAttribute(k_fx_columns<MODE, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
-    cudaFuncSetAttribute(k_fx_columns<MODE, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
 }
 void fx_init()
 {
@@ -315,10 +195,7 @@ void fx_init()
     fx_line_attrs<5, 3>();
     fx_line_attrs<5, 2>();
     fx_line_attrs<3, 1>();
-    fx_col_attrs<COL_DST>();
-    fx_col_attrs<COL_DCT>();
-    fx_col_attrs<COL_DECOMP>();
-    fx_col_attrs<COL_COMBINE>();
+    fx_columns_init();
 }
 
 }  // namespace ps3d

@@ -11,6 +11,7 @@ struct ps3d_closure;
 
 namespace ps3d {
 
+struct Deriv;
 struct Dims {
     int nx, ny, nz;
     int P;                // padded column pitch (>= nz+1, multiple of 8)
@@ -90,6 +91,18 @@ void fx_lines(cudaStream_t st, const double *in, double *out, int n, int P, int 
 // nf consecutive fields (nfield apart) in one launch
 void fx_columns(const Dims &d, cudaStream_t st, int mode, const double *in, double *out, const double *phim,
                 const double *phip, const void *tw, int nf);
+void fx_columns_init();
+// the column work of the FP64 vor2vel and source (fxcol64.cu): cs =
+// combine(c) with es = decompose(central_diffz(cs)); w and dw/dz from the
+// state components; the tendency components of five consecutive transformed
+// products, decomposed
+void fx_comdec(const Dims &d, cudaStream_t st, const double *c, double *cs, double *es, double dzi,
+               const double *phim, const double *phip, const void *tw);
+void fx_w(const Dims &d, cudaStream_t st, const double *A, const double *B, double *w, double *es,
+          const struct Deriv &D, const double *thetam, const double *thetap, const double *dthetam,
+          const double *dthetap, const double *green, const double *rkz, const void *tw);
+void fx_src(const Dims &d, cudaStream_t st, const double *f, double *out, const struct Deriv &D, const double *phim,
+            const double *phip, const void *tw);
 // FP32 bandwidth-tuned line FFTs (lines32.cu), n = 64..1024
 bool lines32_supported(int n);
 void lines32_init();

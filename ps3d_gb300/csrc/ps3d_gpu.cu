@@ -269,6 +269,14 @@ void populate(void *p, size_t bytes)
     const size_t page = (size_t)sysconf(_SC_PAGESIZE);
     char *a = (char *)(((uintptr_t)p + page - 1) / page * page);
     char *e = (char *)(((uintptr_t)p + bytes) / page * page);
+    // an array that was written before has its pages: 16 of them tell
+    bool fresh = false;
+    for (int i = 0; i < 16 && !fresh; ++i) {
+        unsigned char in = 1;
+        char *q = a + (size_t)(e - a - 1) / 16 * i / page * page;
+        fresh = mincore(q, page, &in) != 0 || !(in & 1);
+    }
+    if (!fresh) return;
     std::atomic<size_t> next{0};
     const auto work = [&] {
         for (size_t o; (o = next.fetch_add(PART)) < (size_t)(e - a);) {
@@ -382,6 +390,21 @@ double *scratch64(ps3d_gpu_ctx *c, int i)
     return c->svorf + (size_t)i * c->d.nfield;
 }
 
+// es = decompose(diffz(cs)), cs = combine(C) (inversion.f90:41-47)
+void combine_diffz64(ps3d_gpu_ctx *c, const double *Cc, double *cs, double *es)
+{
+    const Dims &d = c->d;
+    if (fx_serves(d.nz)) {
+        fx_comdec(d, c->st, Cc, cs, es, c->dzi, c->phim64, c->phip64, c->twz2_64);
+        c->launches += 1;
+        return;
+    }
+    columns<double>(d, c->st, COL_COMBINE, Cc, cs, c->phim64, c->phip64, c->twz2_64, nullptr);
+    op_diffz<double>(d, c->st, c->dzi, cs, es);
+    columns<double>(d, c->st, COL_DECOMP, es, es, c->phim64, c->phip64, c->twz2_64, nullptr);
+    c->launches += 3;
+}
+
 // Solenoidal projection of the prognostic vorticity in FP64
 // (inversion.f90:34-76): ds = B_x - A_y, es = decompose(diffz(combine(C))),
 // A = k2l2i (es_x + ds_y), B = k2l2i (es_y - ds_x), (0,0) column kept.
@@ -392,11 +415,9 @@ void project64(ps3d_gpu_ctx *c)
     double *A = c->svor, *B = c->svor + N, *Cc = c->svor + 2 * N;
     double *cs = scratch64(c, 0), *es = scratch64(c, 1), *ds = scratch64(c, 2);
     op_v2v_ds<double, double>(d, c->st, c->D(), A, B, ds);
-    columns<double>(d, c->st, COL_COMBINE, Cc, cs, c->phim64, c->phip64, c->twz2_64, nullptr);
-    op_diffz<double>(d, c->st, c->dzi, cs, es);
-    columns<double>(d, c->st, COL_DECOMP, es, es, c->phim64, c->phip64, c->twz2_64, nullptr);
+    combine_diffz64(c, Cc, cs, es);
     op_v2v_project<double, double>(d, c->st, c->D(), c->k2l2i, es, ds, A, B);
-    c->launches += 5;
+    c->launches += 2;
 }
 
 // FP32 copy of the prognostic state for the mixed form's vor2vel
@@ -436,11 +457,9 @@ int vor2vel_fp64(ps3d_gpu_ctx *c)
 
     // solenoidal projection (inversion.f90:34-76)
     op_v2v_ds<T, double>(d, c->st, D, A, B, ds);
-    col<T>(c, COL_COMBINE, Cc, cs);
-    op_diffz<T>(d, c->st, c->dzi, cs, es);
-    col<T>(c, COL_DECOMP, es, es);
+    combine_diffz64(c, Cc, cs, es);
     op_v2v_project<T, double>(d, c->st, D, c->k2l2i, es, ds, A, B);
-    c->launches += 3;
+    c->launches += 2;
 
     // vorticity in physical space (field_combine_physical x3, :80-82): the
     // first two components combined straight into vor, x lines of those in
@@ -452,16 +471,23 @@ int vor2vel_fp64(ps3d_gpu_ctx *c)
     c->launches += line_launches<T>(c, d.nx, 2) + line_launches<T>(c, d.nx, 1) + line_launches<T>(c, d.ny, 3);
 
     // vertical velocity (:86-139)
-    op_v2v_wsrc<T, double>(d, c->st, D, A, B, ds);
-    op_v2v_wprep<T>(d, c->st, ds, tf<T>(c->thetam), tf<T>(c->thetap), tf<T>(c->dthetam), tf<T>(c->dthetap),
-                    tf<T>(c->green), c->rkz, bs, es, dsg, as);
-    col<T>(c, COL_DCT, as, as);
-    col<T>(c, COL_DST, dsg, dsg);
-    op_v2v_wfinish<T>(d, c->st, dsg, bs, as, svel + 2 * N, es);
+    if (fx_serves(d.nz)) {
+        fx_w(d, c->st, A, B, svel + 2 * N, es, D, tf<T>(c->thetam), tf<T>(c->thetap), tf<T>(c->dthetam),
+             tf<T>(c->dthetap), tf<T>(c->green), c->rkz, c->twz2);
+        c->launches += 1;
+    } else {
+        op_v2v_wsrc<T, double>(d, c->st, D, A, B, ds);
+        op_v2v_wprep<T>(d, c->st, ds, tf<T>(c->thetam), tf<T>(c->thetap), tf<T>(c->dthetam), tf<T>(c->dthetap),
+                        tf<T>(c->green), c->rkz, bs, es, dsg, as);
+        col<T>(c, COL_DCT, as, as);
+        col<T>(c, COL_DST, dsg, dsg);
+        op_v2v_wfinish<T>(d, c->st, dsg, bs, as, svel + 2 * N, es);
+        c->launches += 3;
+    }
     // mean flow (:150-165) and u, v (:169-213)
     op_v2v_meanflow<double>(d, c->st, A, B, c->tables(), c->ubar, c->vbar);
     op_v2v_uv<T>(d, c->st, D, c->k2l2i, es, cs, c->ubar, c->vbar, svel, svel + N);
-    c->launches += 5;
+    c->launches += 2;
     xyi<T>(c, svel, vel, 3);
     return check(c, "vor2vel");
 }
@@ -780,9 +806,16 @@ template <typename T> int source(ps3d_gpu_ctx *c)
     // FP64: as above, assembled before the decomposition (the five products
     // are consecutive); the closure's correction comes decomposed
     xyf<T>(c, r, r, 5);
-    op_svorts<T>(d, c->st, c->D(), r, q, p, gq, gp, svorts, svorts + N, svorts + 2 * N);
-    c->launches += 1;
-    if constexpr (sizeof(T) == sizeof(double)) col64(c, COL_DECOMP, svorts, svorts, 3);
+    if constexpr (sizeof(T) == sizeof(double)) {
+        if (fx_serves(d.nz)) {
+            fx_src(d, c->st, r, svorts, c->D(), tf<T>(c->phim), tf<T>(c->phip), c->twz2);
+            c->launches += 1;
+        } else {
+            op_svorts<T>(d, c->st, c->D(), r, q, p, gq, gp, svorts, svorts + N, svorts + 2 * N);
+            c->launches += 1;
+            col64(c, COL_DECOMP, svorts, svorts, 3);
+        }
+    }
     if (c->closure) closure_add<T>(c, svorts);
     return check(c, "source");
 }
