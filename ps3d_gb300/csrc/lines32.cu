@@ -122,6 +122,43 @@ __device__ __forceinline__ void pass(float4 *sm, const float4 *__restrict__ gin,
     __syncthreads();
 }
 
+// Which levels and lines a block takes.  nz + 1 levels of a power of two nz
+// leave one level to the last 32-level tile, so where at most 8 levels are
+// left a block takes those of four line sets (batches) instead: its row of
+// 32 floats is 4 x 8 levels, 32 bytes of each.  Blocks are numbered z-tile
+// fastest, the tail blocks last.  5 tiles per batch become 4.25 at 128
+// levels: captured 128^3 step 1.271 -> 1.256 ms, batch of twelve runs
+// 88.5 -> 85.9 ms; at 512 levels 17 become 16.25, within the noise.
+struct Tile {
+    int z0;           // first level
+    long long batch;  // (first) batch
+    bool tail;
+    // float offset of quad q (0..7) from the tile's first float, its first
+    // level, and whether its batch exists
+    __device__ long long off(int q, long long bs) const { return tail ? (q >> 1) * bs + 4 * (q & 1) : 4 * q; }
+    __device__ int level(int q) const { return z0 + (tail ? 4 * (q & 1) : 4 * q); }
+    __device__ bool has(int q, long long nbatch) const { return !tail || batch + (q >> 1) < nbatch; }
+};
+struct Tiling {
+    int full;          // 32-level tiles per batch
+    long long nbatch;
+    __host__ __device__ static bool short_tail(int zv) { return zv % 32 >= 1 && zv % 32 <= 8 && zv > 32; }
+    static Tiling of(int zv, long long nbatch) { return Tiling{short_tail(zv) ? zv / 32 : (zv + 31) / 32, nbatch}; }
+    unsigned blocks(int zv) const
+    {
+        return (unsigned)(full * nbatch + (short_tail(zv) ? (nbatch + 3) / 4 : 0));
+    }
+    __device__ Tile tile(unsigned b) const
+    {
+        const unsigned n = (unsigned)(full * nbatch);
+        if (b < n) {
+            const unsigned batch = b / (unsigned)full;
+            return Tile{(int)(b - batch * full) * 2 * LANES, batch, false};
+        }
+        return Tile{full * 2 * LANES, 4ll * (b - n), true};
+    }
+};
+
 // C_k = A_k + i B_k of the two packed lines from the Hermitian rows
 // lo = H[min(k, N-k)] and hi = H[max(k, N-k)] (stafft.f90:55-58 storage)
 __device__ __forceinline__ float2 herm_low(float2 lo, float2 hi) { return make_float2(lo.x - hi.y, hi.x + lo.y); }
@@ -134,8 +171,8 @@ __device__ __forceinline__ float2 herm_high(float2 lo, float2 hi) { return make_
 // its own mirror) for one lane, so every row is loaded once and used for
 // both C_k and C_{N-k}.  Items: slots x 16 lanes over the block's threads.
 template <int N, int W>
-__device__ __forceinline__ void herm_first_pass(float2 *sm2, const float2 *__restrict__ gin2, long long gs2,
-                                                int z0, int P, int zv)
+__device__ __forceinline__ void herm_first_pass(float2 *sm2, const float *__restrict__ in, long long gs2, Tile t,
+                                                long long bs, long long nbatch, int P, int zv)
 {
     constexpr int T = LinePlan<N, true, W>::T, NB = N / 8, SLOTS = NB / 2;
     constexpr int ITEMS = SLOTS * LANES, IPT = (ITEMS + T - 1) / T;
@@ -144,8 +181,9 @@ __device__ __forceinline__ void herm_first_pass(float2 *sm2, const float2 *__res
         const int it = threadIdx.x + T * q;
         if (!(ITEMS % T == 0 || it < ITEMS)) continue;
         const int lane = it & (LANES - 1), s = it / LANES;
-        const bool valid = z0 + 2 * lane < P;
-        const float2 *g = gin2 + lane;
+        const int z = t.level(lane >> 1) + 2 * (lane & 1);
+        const bool valid = z < P && t.has(lane >> 1, nbatch);
+        const float2 *g = reinterpret_cast<const float2 *>(in + t.off(lane >> 1, bs)) + (lane & 1);
         const int j1 = s == 0 ? 0 : s, j2 = s == 0 ? NB / 2 : NB - s;
         float2 h1[8], h2[8];
 #pragma unroll
@@ -154,7 +192,7 @@ __device__ __forceinline__ void herm_first_pass(float2 *sm2, const float2 *__res
             h2[r] = valid ? g[(j2 + r * NB) * gs2] : make_float2(0.f, 0.f);
         }
         // padding rows (z >= zv) enter as zero
-        const int nv = zv - (z0 + 2 * lane);
+        const int nv = zv - z;
         if (nv < 2) {
 #pragma unroll
             for (int r = 0; r < 8; ++r) {
@@ -229,8 +267,9 @@ __device__ __forceinline__ void later_passes(float4 *sm, float4 *gout, long long
 
 template <int N, bool INV, int W>
 __global__ void __launch_bounds__(LinePlan<N, INV, W>::T, LinePlan<N, INV, W>::MINB)
-    k_lines32(const float *__restrict__ in, float *__restrict__ out, int P, int zv, long long line_stride,
-              long long batch_stride, const float2 *__restrict__ tw, long long fs_in, long long fs_out)
+    k_lines32(const float *__restrict__ in, float *__restrict__ out, Tiling tiling, int P, int zv,
+              long long line_stride, long long batch_stride, const float2 *__restrict__ tw, long long fs_in,
+              long long fs_out)
 {
     extern __shared__ __align__(16) float4 smL[];
     // several fields per launch: field blockIdx.z at in + z fs_in, out + z fs_out
@@ -238,37 +277,38 @@ __global__ void __launch_bounds__(LinePlan<N, INV, W>::T, LinePlan<N, INV, W>::M
     out += blockIdx.z * fs_out;
     constexpr int T = LinePlan<N, INV, W>::T;
     const int p = threadIdx.x & (PAIRS - 1);
-    const int z0 = blockIdx.x * 2 * LANES;
-    const bool valid = z0 + 4 * p < P;  // P is a multiple of 8: both lanes or neither
-    const long long base = (long long)blockIdx.y * batch_stride + z0;  // floats
+    const Tile t = tiling.tile(blockIdx.x);
+    const int zt = t.level(p);
+    const bool valid = zt < P && t.has(p, tiling.nbatch);  // P is a multiple of 8: both lanes or neither
+    const long long base = t.batch * batch_stride + t.z0;  // floats
+    const long long mine = base + t.off(p, batch_stride);
     const float s = rsqrtf((float)N);
     constexpr int H = N / 2;
+    const long long gs = line_stride >> 2;  // float4 units
     if (!INV) {
-        const long long gs = line_stride >> 2;  // float4 units
-        const float4 *gin = reinterpret_cast<const float4 *>(in + base) + p;
-        pass<N, 8, 1, false, W, true, false>(smL, gin, nullptr, gs, valid, 1.0f, tw, zv - (z0 + 4 * p));
+        const float4 *gin = reinterpret_cast<const float4 *>(in + mine);
+        pass<N, 8, 1, false, W, true, false>(smL, gin, nullptr, gs, valid, 1.0f, tw, zv - zt);
         later_passes<N, false, W, false>(smL, nullptr, gs, valid, 1.0f, tw);
+        if (!valid) return;
         // split the two packed real transforms of each lane and store the
-        // Hermitian rows k and N - k
-        float4 *o = reinterpret_cast<float4 *>(out + base);
-        for (int e = threadIdx.x; e < (H + 1) * PAIRS; e += T) {
-            const int k = e / PAIRS, q = e & (PAIRS - 1);
-            if (z0 + 4 * q >= P) continue;
-            const float4 ck = smL[k * PAIRS + q];
-            const float4 cn = smL[((N - k) & (N - 1)) * PAIRS + q];
+        // Hermitian rows k and N - k (T is a multiple of PAIRS: every
+        // thread stays on its quad)
+        float4 *o = reinterpret_cast<float4 *>(out + mine);
+        for (int k = threadIdx.x / PAIRS; k <= H; k += T / PAIRS) {
+            const float4 ck = smL[k * PAIRS + p];
+            const float4 cn = smL[((N - k) & (N - 1)) * PAIRS + p];
             // lane 0 in (x, y), lane 1 in (z, w); A = real line z, B = z + 1
             const float4 re = make_float4(0.5f * (ck.x + cn.x) * s, 0.5f * (ck.y + cn.y) * s,
                                           0.5f * (ck.z + cn.z) * s, 0.5f * (ck.w + cn.w) * s);
-            o[k * gs + q] = re;
+            o[k * gs] = re;
             if (k > 0 && k < H)
-                o[(N - k) * gs + q] = make_float4(0.5f * (ck.y - cn.y) * s, -0.5f * (ck.x - cn.x) * s,
-                                                  0.5f * (ck.w - cn.w) * s, -0.5f * (ck.z - cn.z) * s);
+                o[(N - k) * gs] = make_float4(0.5f * (ck.y - cn.y) * s, -0.5f * (ck.x - cn.x) * s,
+                                              0.5f * (ck.w - cn.w) * s, -0.5f * (ck.z - cn.z) * s);
         }
     } else {
-        herm_first_pass<N, W>(reinterpret_cast<float2 *>(smL), reinterpret_cast<const float2 *>(in + base),
-                              line_stride >> 1, z0, P, zv);
-        const long long gs = line_stride >> 2;
-        float4 *gout = reinterpret_cast<float4 *>(out + base) + p;
+        herm_first_pass<N, W>(reinterpret_cast<float2 *>(smL), in + base, line_stride >> 1, t, batch_stride,
+                              tiling.nbatch, P, zv);
+        float4 *gout = reinterpret_cast<float4 *>(out + mine);
         later_passes<N, true, W, true>(smL, gout, gs, valid, s, tw);
     }
 }
@@ -277,9 +317,10 @@ template <int N, bool INV, int W>
 void launch32w(cudaStream_t st, const float *in, float *out, int P, int zv, long long ls, long long nbatch,
                long long bs, const float2 *tw, int nf, long long fs_in, long long fs_out)
 {
-    dim3 grid((P + 2 * LANES - 1) / (2 * LANES), (unsigned)nbatch, (unsigned)nf);
+    const Tiling tiling = Tiling::of(zv, nbatch);
+    const dim3 grid(tiling.blocks(zv), 1, (unsigned)nf);
     const size_t sm = (size_t)N * LANES * sizeof(float2);
-    k_lines32<N, INV, W><<<grid, LinePlan<N, INV, W>::T, sm, st>>>(in, out, P, zv, ls, bs, tw, fs_in, fs_out);
+    k_lines32<N, INV, W><<<grid, LinePlan<N, INV, W>::T, sm, st>>>(in, out, tiling, P, zv, ls, bs, tw, fs_in, fs_out);
 }
 
 
@@ -311,8 +352,8 @@ struct ProdSrc {
 
 template <int N, int W>
 __global__ void __launch_bounds__(LinePlan<N, false, W>::T, LinePlan<N, false, W>::MINB)
-    k_lines32_prod(ProdSrc ps, float *__restrict__ out, int P, long long line_stride, long long batch_stride,
-                   const float2 *__restrict__ tw)
+    k_lines32_prod(ProdSrc ps, float *__restrict__ out, Tiling tiling, int P, long long line_stride,
+                   long long batch_stride, const float2 *__restrict__ tw)
 {
     extern __shared__ __align__(16) float4 smL[];
     constexpr int T = LinePlan<N, false, W>::T, G = LinePlan<N, false, W>::G;
@@ -322,11 +363,13 @@ __global__ void __launch_bounds__(LinePlan<N, false, W>::T, LinePlan<N, false, W
     // shuffles below always run on full warps
     static_assert(NB % 4 == 0 && PAIRS == 8, "warp-uniform butterfly ranges");
     const int o = blockIdx.x % 3;
-    const int z0 = (blockIdx.x / 3) * 2 * LANES;
+    const Tile t = tiling.tile(blockIdx.x / 3);
     const int p = threadIdx.x & (PAIRS - 1), g = threadIdx.x / PAIRS;
-    const int zt = z0 + 4 * p;  // first of the thread's four levels
-    const bool valid = zt < P;  // P is a multiple of 8: all four or none
-    const long long base = (long long)blockIdx.y * batch_stride + z0;
+    const int zt = t.level(p);  // first of the thread's four levels
+    const bool valid = zt < P && t.has(p, tiling.nbatch);  // P is a multiple of 8: all four or none
+    // first and last quad of a run of levels: their outer neighbours are loaded
+    const bool first = t.tail ? !(p & 1) : p == 0, last = t.tail ? (p & 1) : p == PAIRS - 1;
+    const long long base = t.batch * batch_stride + t.z0 + t.off(p, batch_stride);
     const long long Nf = ps.nfield;
     const float *u = ps.vel, *v = ps.vel + Nf, *w = ps.vel + 2 * Nf;
     const float *xi = ps.vor, *eta = ps.vor + Nf, *zeta = ps.vor + 2 * Nf;
@@ -368,15 +411,15 @@ __global__ void __launch_bounds__(LinePlan<N, false, W>::T, LinePlan<N, false, W
     // the product at (row, levels zt..zt+3); blocks 1, 2 write its z
     // derivative there to their derivative's output tile
     auto load = [&](int row) -> float4 {
-        const long long i = base + (long long)row * line_stride + 4 * p;
+        const long long i = base + (long long)row * line_stride;
         const float4 f = valid ? prod4(i) : make_float4(0.f, 0.f, 0.f, 0.f);
         if (o) {
             // neighbours zt - 1 and zt + 4: from the threads beside this one
             // in the row, or loaded at the block's edges
             float fm = __shfl_up_sync(0xffffffffu, f.w, 1);
             float fp = __shfl_down_sync(0xffffffffu, f.x, 1);
-            if (p == 0) fm = (valid && zt > 0) ? prod(i - 1) : 0.f;
-            if (p == PAIRS - 1) fp = (valid && zt + 4 <= nz) ? prod(i + 4) : 0.f;
+            if (first) fm = (valid && zt > 0) ? prod(i - 1) : 0.f;
+            if (last) fp = (valid && zt + 4 <= nz) ? prod(i + 4) : 0.f;
             const float lv[6] = {fm, f.x, f.y, f.z, f.w, fp};
             float dv[4];
 #pragma unroll
@@ -396,18 +439,17 @@ __global__ void __launch_bounds__(LinePlan<N, false, W>::T, LinePlan<N, false, W
     // split the two packed real transforms of each lane, store the
     // Hermitian rows k and N - k (as k_lines32)
     auto store = [&](float *dst) {
+        if (!valid) return;
         float4 *ob = reinterpret_cast<float4 *>(dst + base);
-        for (int e = threadIdx.x; e < (H + 1) * PAIRS; e += T) {
-            const int k = e / PAIRS, q = e & (PAIRS - 1);
-            if (z0 + 4 * q >= P) continue;
-            const float4 ck = smL[k * PAIRS + q];
-            const float4 cn = smL[((N - k) & (N - 1)) * PAIRS + q];
+        for (int k = g; k <= H; k += T / PAIRS) {
+            const float4 ck = smL[k * PAIRS + p];
+            const float4 cn = smL[((N - k) & (N - 1)) * PAIRS + p];
             const float4 re = make_float4(0.5f * (ck.x + cn.x) * s, 0.5f * (ck.y + cn.y) * s,
                                           0.5f * (ck.z + cn.z) * s, 0.5f * (ck.w + cn.w) * s);
-            ob[k * gs + q] = re;
+            ob[k * gs] = re;
             if (k > 0 && k < H)
-                ob[(N - k) * gs + q] = make_float4(0.5f * (ck.y - cn.y) * s, -0.5f * (ck.x - cn.x) * s,
-                                                   0.5f * (ck.w - cn.w) * s, -0.5f * (ck.z - cn.z) * s);
+                ob[(N - k) * gs] = make_float4(0.5f * (ck.y - cn.y) * s, -0.5f * (ck.x - cn.x) * s,
+                                               0.5f * (ck.w - cn.w) * s, -0.5f * (ck.z - cn.z) * s);
         }
     };
     // first radix-8 pass (span 1) of the product: butterfly j reads rows
@@ -443,7 +485,7 @@ __global__ void __launch_bounds__(LinePlan<N, false, W>::T, LinePlan<N, false, W
     // the derivative: each thread reads back the values it parked (its own
     // rows and levels), then the same transform in place
     __syncthreads();
-    const float4 *gin = reinterpret_cast<const float4 *>(dout + base) + p;
+    const float4 *gin = reinterpret_cast<const float4 *>(dout + base);
     pass<N, 8, 1, false, W, true, false>(smL, gin, nullptr, gs, valid, 1.0f, tw, nval);
     later_passes<N, false, W, false>(smL, nullptr, gs, valid, 1.0f, tw);
     store(dout);
@@ -452,10 +494,10 @@ __global__ void __launch_bounds__(LinePlan<N, false, W>::T, LinePlan<N, false, W
 template <int N, int W>
 void launch_prod(cudaStream_t st, const ProdSrc &ps, float *out, int P, int nx, int ny, const float2 *tw)
 {
-    const int ztiles = (P + 2 * LANES - 1) / (2 * LANES);
-    dim3 grid((unsigned)(3 * ztiles), (unsigned)nx);
+    const Tiling tiling = Tiling::of(ps.nz + 1, nx);
     const size_t sm = (size_t)N * LANES * sizeof(float2);
-    k_lines32_prod<N, W><<<grid, LinePlan<N, false, W>::T, sm, st>>>(ps, out, P, P, (long long)ny * P, tw);
+    k_lines32_prod<N, W><<<3 * tiling.blocks(ps.nz + 1), LinePlan<N, false, W>::T, sm, st>>>(
+        ps, out, tiling, P, P, (long long)ny * P, tw);
 }
 
 // ------------------------------------------------------------------------
