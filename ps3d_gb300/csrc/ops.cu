@@ -311,9 +311,11 @@ void op_products(const Dims &d, cudaStream_t st, const T *vel, const T *vor, T *
 // The products together with the z derivatives of q and p (central_diffz,
 // inversion_utils.f90:653-673) in one pass over each column: the
 // neighbours iz -+ 1 come from the adjacent lanes, and across 32-level
-// chunks from the previous chunk (carried) or the next one (the last lane's
-// derivative is written one chunk later).  Same arithmetic as k_products
-// followed by k_diffz.
+// chunks from the previous chunk (carried) or the next one, whose products
+// are formed before this chunk's derivatives.  One difference and one
+// product per derivative for all lanes alike: lane-dependent branches cost
+// the FP64 form a pass of its pipe each (256^3: 754 us with them, 361 now).  Same
+// arithmetic as k_products followed by k_diffz.
 template <typename T>
 __global__ void k_products_dz(Dims d, T dzi, T hdzi, const T *__restrict__ vel, const T *__restrict__ vor,
                               T *__restrict__ r, T *__restrict__ q, T *__restrict__ p, T *__restrict__ gq,
@@ -322,56 +324,55 @@ __global__ void k_products_dz(Dims d, T dzi, T hdzi, const T *__restrict__ vel, 
     COLUMN_HEADER
     const long long N = d.nfield;
     const int nz = d.nz, lane = threadIdx.x;
-    T q1 = 0, p1 = 0, q2 = 0, p2 = 0;  // levels 32c - 1 and 32c - 2 of the previous chunk
+    // products of level iz, stored; 0 above the top wall
+    const auto products = [&](int iz, T &qv, T &pv) {
+        qv = pv = 0;
+        if (iz > nz) return;
+        const long long i = o + iz;
+        const T u = vel[i], v = vel[N + i], w = vel[2 * N + i];
+        const T xi = vor[i], eta = vor[N + i], zeta = vor[2 * N + i];
+        r[i] = u * eta - v * xi;
+        qv = w * xi - u * zeta;
+        pv = v * zeta - w * eta;
+        q[i] = qv;
+        p[i] = pv;
+    };
+    T qv, pv, q1 = 0, p1 = 0;  // this chunk, and the level below it
+    products(lane, qv, pv);
     for (int c0 = 0; c0 <= nz; c0 += 32) {
         const int iz = c0 + lane;
-        T qv = 0, pv = 0;
-        if (iz <= nz) {
-            const long long i = o + iz;
-            const T u = vel[i], v = vel[N + i], w = vel[2 * N + i];
-            const T xi = vor[i], eta = vor[N + i], zeta = vor[2 * N + i];
-            r[i] = u * eta - v * xi;
-            qv = w * xi - u * zeta;
-            pv = v * zeta - w * eta;
-            q[i] = qv;
-            p[i] = pv;
-        }
+        T qx, px;  // the next chunk
+        products(iz + 32, qx, px);
         T qm = __shfl_up_sync(0xffffffffu, qv, 1), pm = __shfl_up_sync(0xffffffffu, pv, 1);
-        const T qn = __shfl_down_sync(0xffffffffu, qv, 1), pn = __shfl_down_sync(0xffffffffu, pv, 1);
-        const T q0 = __shfl_sync(0xffffffffu, qv, 0), p0 = __shfl_sync(0xffffffffu, pv, 0);
+        T qn = __shfl_down_sync(0xffffffffu, qv, 1), pn = __shfl_down_sync(0xffffffffu, pv, 1);
+        const T q0 = __shfl_sync(0xffffffffu, qx, 0), p0 = __shfl_sync(0xffffffffu, px, 0);
+        const bool bottom = iz == 0, top = iz == nz;
         if (lane == 0) {
             qm = q1;
             pm = p1;
         }
-        // the previous chunk's last level, now that its upper neighbour is known
-        if (c0 > 0 && lane == 31) {
-            gq[o + c0 - 1] = (q0 - q2) * hdzi;
-            gp[o + c0 - 1] = (p0 - p2) * hdzi;
+        if (lane == 31) {
+            qn = q0;
+            pn = p0;
         }
+        if (bottom) {
+            qm = qv;
+            pm = pv;
+        }
+        if (top) {
+            qn = qv;
+            pn = pv;
+        }
+        const T s = bottom || top ? dzi : hdzi;
+        const T a = (qn - qm) * s, b = (pn - pm) * s;
         if (iz <= nz) {
-            T a = 0, b = 0;
-            bool put = true;
-            if (iz == 0) {
-                a = (qn - qv) * dzi;
-                b = (pn - pv) * dzi;
-            } else if (iz == nz) {
-                a = (qv - qm) * dzi;
-                b = (pv - pm) * dzi;
-            } else if (lane < 31) {
-                a = (qn - qm) * hdzi;
-                b = (pn - pm) * hdzi;
-            } else {
-                put = false;
-            }
-            if (put) {
-                gq[o + iz] = a;
-                gp[o + iz] = b;
-            }
+            gq[o + iz] = a;
+            gp[o + iz] = b;
         }
         q1 = __shfl_sync(0xffffffffu, qv, 31);
         p1 = __shfl_sync(0xffffffffu, pv, 31);
-        q2 = __shfl_sync(0xffffffffu, qv, 30);
-        p2 = __shfl_sync(0xffffffffu, pv, 30);
+        qv = qx;
+        pv = px;
     }
 }
 template <typename T>
