@@ -63,8 +63,8 @@ static_assert(NPARAM == PS3D_CLOSURE_NPARAM, "parameter count");
 
 constexpr int CONV_THREADS = 128;  // 4 warps
 constexpr int CONV_ROWS = 128;     // grid points per block tile (32 per warp)
-constexpr int WG_KW = 32;          // 16-point k steps per warp in the weight gradient
-constexpr int WG_CHUNK = 4 * WG_KW * 16;
+constexpr int WG_SEG = 512;        // points per partial sum of the weight gradient
+constexpr int WG_CHUNK = 4 * WG_SEG;
 constexpr int RED_THREADS = 256;
 constexpr int RED_BLOCKS = 256;
 
@@ -264,93 +264,165 @@ __global__ void __launch_bounds__(CONV_THREADS, 4) k_conv(ConvArgs a)
 
 // Weight gradient of one layer, partial sums per chunk of WG_CHUNK points:
 // part[chunk][tap][ci][co] = sum_p X_tap[p][ci] dZ[p][co], tap 27 = bias.
-template <int CIN, int COUT>
-__global__ void __launch_bounds__(128) k_wgrad(const bf16 *__restrict__ act, const bf16 *__restrict__ dz,
-                                               float *__restrict__ part, int nx, int ny, int Z, long long npts)
+//
+// One block per chunk takes all 27 taps.  Its stages of 128 points come by
+// asynchronous copies into two buffers: the dZ rows once, and for each of the
+// nine neighbour columns (dx, dy) the run of X rows with one row more at each
+// end, which serves the three dz taps.  Warp (dx, dy, m) keeps the products of
+// its three taps and 16 input channels in registers; a dz tap that would leave
+// the grid through a wall meets dZ fragments whose rows there are zero (a mask
+// per row).  The last warp multiplies by ones: the bias.  A block per tap and
+// chunk read the same rows 28 times, and index arithmetic and staging, not the
+// tensor pipe, took its time: 32 -> 32 channels at 64^3 219 us, 99 us here, where the warp-level
+// products (about 240 TFLOP/s at most on this chip) bound it.
+// Segments of 512 points are summed in the order of the four warps that took
+// one each there, so the sums are bitwise those.
+template <int CIN, int COUT> struct WG {
+    static constexpr int MT = CIN / 16, NT = COUT / 8, WARPS = 9 * MT + 1, THREADS = 32 * WARPS;
+    static constexpr int L = 128, XROWS = L + 2;
+    static constexpr int XS = CIN * 2 + 16, GS = COUT * 2 + 16;  // padded rows: conflict-free ldmatrix
+    static constexpr int XB = 9 * XROWS * XS, GB = L * GS, MB = 2 * L * 2, TB = XROWS * 16;
+    static constexpr int BUF = XB + GB + MB + TB;
+    static_assert(WG_SEG % L == 0 && WG_CHUNK == 4 * WG_SEG && BUF % 16 == 0, "stage layout");
+};
+__device__ __forceinline__ void copy16(void *dst, const void *src, bool on)
 {
-    constexpr int XS = CIN * 2 + 16;  // padded row bytes: conflict-free ldmatrix
-    constexpr int GS = COUT * 2 + 16;
-    constexpr int MT = CIN / 16, NT = COUT / 8;
-    __shared__ __align__(16) unsigned char sx[4][16 * XS];
-    __shared__ __align__(16) unsigned char sg[4][16 * GS];
-    __shared__ float red[4][CIN * COUT];
-    const int tap = blockIdx.y;
-    const long long chunk = blockIdx.x;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int g = lane >> 2, t = lane & 3;
-    const int dx = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dzz = tap % 3 - 1;
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(on ? 16 : 0) : "memory");
+}
+template <int CIN, int COUT>
+__global__ void __launch_bounds__(WG<CIN, COUT>::THREADS, 1)
+    k_wgrad(const bf16 *__restrict__ act, const bf16 *__restrict__ dz, float *__restrict__ part, int nx, int ny, int Z,
+            long long npts)
+{
+    using C = WG<CIN, COUT>;
+    constexpr int NT = C::NT, L = C::L, XROWS = C::XROWS, XS = C::XS, GS = C::GS;
+    extern __shared__ __align__(16) unsigned char smw[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int g = lane >> 2, t = lane & 3, mi = lane >> 3, mr = lane & 7;
     const int nym = ny - 1, nxm = nx - 1;
-    float acc[MT][NT][4];
+    const bool bias = warp == C::WARPS - 1;
+    const int dxy = bias ? 0 : warp / C::MT, m = bias ? 0 : warp % C::MT;
+    const long long c0 = (long long)blockIdx.x * WG_CHUNK;
+    float acc[3][NT][4];
 #pragma unroll
-    for (int m = 0; m < MT; ++m)
+    for (int d = 0; d < 3; ++d)
 #pragma unroll
         for (int n = 0; n < NT; ++n)
 #pragma unroll
-            for (int q = 0; q < 4; ++q) acc[m][n][q] = 0.f;
+            for (int q = 0; q < 4; ++q) acc[d][n][q] = 0.f;
 
-    const long long p0 = (chunk * 4 + warp) * (long long)(WG_KW * 16);
-    unsigned char *xs = sx[warp];
-    unsigned char *gs = sg[warp];
-    for (int k = 0; k < WG_KW; ++k) {
-        const long long pb = p0 + k * 16;
-        if (pb >= npts) break;  // warp-uniform
-        for (int e = lane; e < 16 * (CIN / 8); e += 32) {
-            const int row = e / (CIN / 8), q = e % (CIN / 8);
-            const long long p = pb + row;
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if (p < npts) {
-                if (tap == NTAP) {
-                    if (q == 0) v.x = 0x3F80u;  // BF16 1.0 in channel 0
-                } else {
-                    const long long col = p / Z;
-                    const int iz = (int)(p - col * Z) + dzz;
-                    if (iz >= 0 && iz < Z) {
-                        const int iy = (int)(col & nym), ix = (int)(col / ny);
-                        const long long pn =
-                            iz + (long long)Z * ((long long)((iy + dy) & nym) + (long long)ny * ((ix + dx) & nxm));
-                        v = __ldg(reinterpret_cast<const uint4 *>(act + pn * CIN) + q);
+    const auto xbuf = [&](int b) { return smw + b * C::BUF; };
+    const auto gbuf = [&](int b) { return smw + b * C::BUF + C::XB; };
+    const auto mask = [&](int b) { return reinterpret_cast<unsigned short *>(smw + b * C::BUF + C::XB + C::GB); };
+    const auto tab = [&](int b) { return reinterpret_cast<int4 *>(smw + b * C::BUF + C::XB + C::GB + C::MB); };
+    // level and column of the rows of a stage (row r is point p0 - 1 + r)
+    const auto rows = [&](long long p0, int b) {
+        for (int r = tid; r < XROWS; r += C::THREADS) {
+            const long long q = p0 - 1 + r;
+            int4 e = make_int4(0, 0, 0, 0);
+            if (q >= 0 && q < npts) {
+                const long long col = q / Z;
+                e = make_int4((int)(q - col * Z), (int)(col & nym), (int)(col / ny), 1);
+            }
+            tab(b)[r] = e;
+            if (r >= 1 && r <= L) {
+                mask(b)[r - 1] = e.x == 0 ? 0 : 0xffff;          // dz = -1
+                mask(b)[L + r - 1] = e.x == Z - 1 ? 0 : 0xffff;  // dz = +1
+            }
+        }
+    };
+    const auto issue = [&](long long p0, int b) {
+        constexpr int C8 = CIN / 8, G8 = COUT / 8;
+        for (int e = tid; e < 9 * XROWS * C8; e += C::THREADS) {
+            const int k = e / (XROWS * C8), rem = e - k * (XROWS * C8), r = rem / C8, q = rem % C8;
+            const int4 w = tab(b)[r];
+            const long long row =
+                w.x + (long long)Z * (((w.y + k % 3 - 1) & nym) + (long long)ny * ((w.z + k / 3 - 1) & nxm));
+            copy16(xbuf(b) + (k * XROWS + r) * XS + q * 16, act + (w.w ? row * CIN : 0) + q * 8, w.w);
+        }
+        for (int e = tid; e < L * G8; e += C::THREADS) {
+            const int r = e / G8, q = e % G8;
+            const bool on = p0 + r < npts;
+            copy16(gbuf(b) + r * GS + q * 16, dz + (on ? (p0 + r) * COUT : 0) + q * 8, on);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // the segment's sums into the partial result (this thread's own places)
+    float *out = part + (long long)blockIdx.x * (NTAP + 1) * (CIN * COUT);
+    const auto flush = [&](bool first) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            if (bias && d) break;
+            float *o = out + (long long)(bias ? NTAP : 3 * dxy + d) * (CIN * COUT);
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    float2 *w = reinterpret_cast<float2 *>(o + (m * 16 + g + 8 * h) * COUT + n * 8 + 2 * t);
+                    float2 v = make_float2(acc[d][n][2 * h], acc[d][n][2 * h + 1]);
+                    if (!first) {
+                        const float2 old = *w;
+                        v = make_float2(old.x + v.x, old.y + v.y);
                     }
+                    *w = v;
+                    acc[d][n][2 * h] = acc[d][n][2 * h + 1] = 0.f;
                 }
-            }
-            *reinterpret_cast<uint4 *>(xs + row * XS + q * 16) = v;
         }
-        for (int e = lane; e < 16 * (COUT / 8); e += 32) {
-            const int row = e / (COUT / 8), q = e % (COUT / 8);
-            const long long p = pb + row;
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if (p < npts) v = __ldg(reinterpret_cast<const uint4 *>(dz + p * COUT) + q);
-            *reinterpret_cast<uint4 *>(gs + row * GS + q * 16) = v;
-        }
-        __syncwarp();
-        const int mi = lane >> 3, mr = lane & 7;
-        uint32_t A[MT][4];
-#pragma unroll
-        for (int m = 0; m < MT; ++m)
-            ldsm_x4_trans(A[m][0], A[m][1], A[m][2], A[m][3],
-                          xs + (mr + 8 * (mi >> 1)) * XS + (m * 16 + 8 * (mi & 1)) * 2);
-        uint32_t B[NT][2];
-#pragma unroll
-        for (int n2 = 0; n2 < NT / 2; ++n2)
-            ldsm_x4_trans(B[2 * n2][0], B[2 * n2][1], B[2 * n2 + 1][0], B[2 * n2 + 1][1],
-                          gs + (mr + 8 * (mi & 1)) * GS + (n2 * 16 + 8 * (mi >> 1)) * 2);
-#pragma unroll
-        for (int m = 0; m < MT; ++m)
-#pragma unroll
-            for (int n = 0; n < NT; ++n) mma16816(acc[m][n], A[m][0], A[m][1], A[m][2], A[m][3], B[n][0], B[n][1]);
-        __syncwarp();
-    }
-#pragma unroll
-    for (int m = 0; m < MT; ++m)
-#pragma unroll
-        for (int n = 0; n < NT; ++n)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const int ci = m * 16 + g + 8 * (q >> 1), co = n * 8 + 2 * t + (q & 1);
-                red[warp][ci * COUT + co] = acc[m][n][q];
-            }
+    };
+
+    constexpr int STAGES = WG_CHUNK / L;
+    rows(c0, 0);
     __syncthreads();
-    float *dst = part + (chunk * (NTAP + 1) + tap) * (long long)(CIN * COUT);
-    for (int e = threadIdx.x; e < CIN * COUT; e += 128) dst[e] = red[0][e] + red[1][e] + red[2][e] + red[3][e];
+    issue(c0, 0);
+    for (int s = 0; s < STAGES; ++s) {
+        const int b = s & 1;
+        const bool more = s + 1 < STAGES && c0 + (long long)(s + 1) * L < npts;
+        if (more) {
+            rows(c0 + (long long)(s + 1) * L, b ^ 1);
+            __syncthreads();
+            issue(c0 + (long long)(s + 1) * L, b ^ 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();
+        const unsigned char *xs = xbuf(b) + dxy * XROWS * XS, *gs = gbuf(b);
+        const unsigned short *mk = mask(b);
+#pragma unroll 2
+        for (int k0 = 0; k0 < L; k0 += 16) {
+            uint32_t B[NT][2];
+#pragma unroll
+            for (int n2 = 0; n2 < NT / 2; ++n2)
+                ldsm_x4_trans(B[2 * n2][0], B[2 * n2][1], B[2 * n2 + 1][0], B[2 * n2 + 1][1],
+                              gs + (k0 + mr + 8 * (mi & 1)) * GS + (n2 * 16 + 8 * (mi >> 1)) * 2);
+            if (bias) {
+                const uint32_t one = g == 0 ? 0x3F803F80u : 0u;  // BF16 ones in channel 0
+#pragma unroll
+                for (int n = 0; n < NT; ++n) mma16816(acc[0][n], one, 0u, one, 0u, B[n][0], B[n][1]);
+                continue;
+            }
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                uint32_t A[4];
+                ldsm_x4_trans(A[0], A[1], A[2], A[3],
+                              xs + (k0 + d + mr + 8 * (mi >> 1)) * XS + (m * 16 + 8 * (mi & 1)) * 2);
+                uint32_t lo = 0xffffffffu, hi = 0xffffffffu;  // rows 2t, 2t + 1 and those 8 further
+                if (d != 1) {
+                    const unsigned short *q = mk + (d == 0 ? 0 : L) + k0 + 2 * t;
+                    lo = *reinterpret_cast<const uint32_t *>(q);
+                    hi = *reinterpret_cast<const uint32_t *>(q + 8);
+                }
+#pragma unroll
+                for (int n = 0; n < NT; ++n)
+                    mma16816(acc[d][n], A[0], A[1], A[2], A[3], B[n][0] & lo, B[n][1] & hi);
+            }
+        }
+        const bool last = !more;
+        if ((s + 1) * L % WG_SEG == 0 || last) flush((s * L) / WG_SEG == 0);
+        if (last) break;
+        __syncthreads();
+    }
 }
 
 // grad[e] for e < 27*cin*cout + cout (weights then bias of one layer)
@@ -369,6 +441,7 @@ __global__ void k_wgrad_reduce(const float *__restrict__ part, long long nchunk,
     }
     const long long stride = (long long)(NTAP + 1) * CIN * COUT;
     float s = 0.f;
+#pragma unroll 8  // the loads of eight chunks at a time, the sum in order
     for (long long c = 0; c < nchunk; ++c) s += part[c * stride + src];
     grad[e] = s;
 }
@@ -1191,8 +1264,8 @@ void forward(ps3d_closure *cl, cudaStream_t st)
 
 template <int CIN, int COUT> void wgrad(ps3d_closure *cl, cudaStream_t st, const bf16 *act, const bf16 *dz, int l)
 {
-    dim3 grid((unsigned)cl->nchunk, NTAP + 1);
-    k_wgrad<CIN, COUT><<<grid, 128, 0, st>>>(act, dz, cl->wpart, cl->nx, cl->ny, cl->Z, cl->npts);
+    k_wgrad<CIN, COUT><<<(unsigned)cl->nchunk, WG<CIN, COUT>::THREADS, 2 * WG<CIN, COUT>::BUF, st>>>(
+        act, dz, cl->wpart, cl->nx, cl->ny, cl->Z, cl->npts);
     const int n = NTAP * CREAL_IN[l] * CREAL_OUT[l] + CREAL_OUT[l];
     k_wgrad_reduce<<<(n + 255) / 256, 256, 0, st>>>(cl->wpart, cl->nchunk, CIN, COUT, CREAL_IN[l], CREAL_OUT[l],
                                                     cl->g + woff(l));
@@ -1379,6 +1452,9 @@ int ps3d_closure_create(int nx, int ny, int nz, int max_samples, int device, uns
     conv_attr<32, 8, EPI_OUT>(cl);
     conv_attr<16, 32, EPI_BWD>(cl);
     conv_attr<32, 32, EPI_BWD>(cl);
+    cudaFuncSetAttribute(k_wgrad<16, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * WG<16, 32>::BUF);
+    cudaFuncSetAttribute(k_wgrad<32, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * WG<32, 32>::BUF);
+    cudaFuncSetAttribute(k_wgrad<32, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * WG<32, 16>::BUF);
     // tcgen05 path: padded geometry; available when a tile's shared memory
     // (weights + 3 x 4 chunk planes of 128 + 2(ZP+1) rows) fits a block
     cl->ZP = nz + 3;
