@@ -21,6 +21,10 @@ struct Dims {
     // [0] forward y, [1] forward x, [2] inverse y, [3] inverse x;
     // -1 = the default shape of the line length
     signed char line_shape[4] = {-1, -1, -1, -1};
+    // FP64 transforms in fixed point (the FP64 form).  The mixed form installs
+    // a state (set-up, set_field, load) with the FP64 Stockham kernels: a
+    // last-bit change there would change every FP32 rounding of the run.
+    bool fx64 = false;
 };
 
 enum { COL_DST = 0, COL_DCT = 1, COL_DECOMP = 2, COL_COMBINE = 3 };

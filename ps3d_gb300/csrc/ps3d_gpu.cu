@@ -123,6 +123,7 @@ struct ps3d_gpu_ctx {
     // FP64 transform tables for the FP64 set-up / projection of the mixed
     // form (aliases of the above in the FP64 form)
     double2 *twx64 = nullptr, *twy64 = nullptr, *twz2_64 = nullptr;
+    void *twz2_fx = nullptr;  // fx_twiddles of 2 nz (the FP64 form: twz2)
     double *phim64 = nullptr, *phip64 = nullptr;
     // per-column and per-level FP64 tables
     double *k2l2 = nullptr, *k2l2i = nullptr, *filt0 = nullptr, *vhdis = nullptr, *vdiss = nullptr;
@@ -322,7 +323,7 @@ int download(ps3d_gpu_ctx *c, const void *src, bool src_is_fp64, int ncomp, doub
 // line kernels, one per field otherwise
 template <typename T> int line_launches(const ps3d_gpu_ctx *c, int n, int nf)
 {
-    return (sizeof(T) == sizeof(float) ? lines32_supported(n) : fx_serves(n)) ? 1 : nf;
+    return (sizeof(T) == sizeof(float) ? lines32_supported(n) : c->d.fx64 && fx_serves(n)) ? 1 : nf;
 }
 // horizontal transforms of nf consecutive fields (nfield apart)
 template <typename T> void xyf(ps3d_gpu_ctx *c, const T *in, T *out, int nf = 1)
@@ -360,7 +361,7 @@ void col64(ps3d_gpu_ctx *c, int mode, const double *in, double *out, int nf)
 {
     columns<double>(c->d, c->st, mode, in, out, tf<double>(c->phim), tf<double>(c->phip), tf<double2>(c->twz2),
                     &c->probe, nf);
-    c->launches += fx_serves(c->d.nz) ? 1 : nf;
+    c->launches += c->d.fx64 && fx_serves(c->d.nz) ? 1 : nf;
 }
 // a T view of an FP64 state component (copy for the mixed form)
 template <typename T> const T *state_as_T(ps3d_gpu_ctx *c, const double *s, T *scratch)
@@ -390,12 +391,13 @@ double *scratch64(ps3d_gpu_ctx *c, int i)
     return c->svorf + (size_t)i * c->d.nfield;
 }
 
-// es = decompose(diffz(cs)), cs = combine(C) (inversion.f90:41-47)
-void combine_diffz64(ps3d_gpu_ctx *c, const double *Cc, double *cs, double *es)
+// es = decompose(diffz(cs)), cs = combine(C) (inversion.f90:41-47).  step:
+// inside a step (vor2vel of the FP64 form, the re-projection of mixed cn2)
+void combine_diffz64(ps3d_gpu_ctx *c, const double *Cc, double *cs, double *es, bool step)
 {
     const Dims &d = c->d;
-    if (fx_serves(d.nz)) {
-        fx_comdec(d, c->st, Cc, cs, es, c->dzi, c->phim64, c->phip64, c->twz2_64);
+    if (step && fx_serves(d.nz)) {
+        fx_comdec(d, c->st, Cc, cs, es, c->dzi, c->phim64, c->phip64, c->twz2_fx);
         c->launches += 1;
         return;
     }
@@ -408,14 +410,14 @@ void combine_diffz64(ps3d_gpu_ctx *c, const double *Cc, double *cs, double *es)
 // Solenoidal projection of the prognostic vorticity in FP64
 // (inversion.f90:34-76): ds = B_x - A_y, es = decompose(diffz(combine(C))),
 // A = k2l2i (es_x + ds_y), B = k2l2i (es_y - ds_x), (0,0) column kept.
-void project64(ps3d_gpu_ctx *c)
+void project64(ps3d_gpu_ctx *c, bool step)
 {
     const Dims &d = c->d;
     const long long N = d.nfield;
     double *A = c->svor, *B = c->svor + N, *Cc = c->svor + 2 * N;
     double *cs = scratch64(c, 0), *es = scratch64(c, 1), *ds = scratch64(c, 2);
     op_v2v_ds<double, double>(d, c->st, c->D(), A, B, ds);
-    combine_diffz64(c, Cc, cs, es);
+    combine_diffz64(c, Cc, cs, es, step);
     op_v2v_project<double, double>(d, c->st, c->D(), c->k2l2i, es, ds, A, B);
     c->launches += 2;
 }
@@ -429,9 +431,9 @@ void refresh32(ps3d_gpu_ctx *c)
 }
 
 // projection of an externally set state, then its FP32 copy (mixed form)
-void project_state_mixed(ps3d_gpu_ctx *c)
+void project_state_mixed(ps3d_gpu_ctx *c, bool step = false)
 {
-    project64(c);
+    project64(c, step);
     refresh32(c);
 }
 
@@ -457,7 +459,7 @@ int vor2vel_fp64(ps3d_gpu_ctx *c)
 
     // solenoidal projection (inversion.f90:34-76)
     op_v2v_ds<T, double>(d, c->st, D, A, B, ds);
-    combine_diffz64(c, Cc, cs, es);
+    combine_diffz64(c, Cc, cs, es, true);
     op_v2v_project<T, double>(d, c->st, D, c->k2l2i, es, ds, A, B);
     c->launches += 2;
 
@@ -1159,7 +1161,7 @@ template <typename T> int step_cn2(ps3d_gpu_ctx *c, double *t, double dt)
     op_cn2_init<T>(d, c->st, c->vortsm, c->svor, sv, dt2);
     op_cn2_update<T>(d, c->st, c->svor, c->vortsm, sv, c->filt0, c->fz, c->vdiss, dt2);
     op_mean_fix(d, c->st, c->svor, c->dstsum, c->fnzi, c->ini, nullptr, 1);
-    if (mixed) project_state_mixed(c);
+    if (mixed) project_state_mixed(c, true);
     c->launches += 7;
     for (int it = 0; it < 2; ++it) {
         int rc = rhs_or_hold<T>(c);
@@ -1171,7 +1173,7 @@ template <typename T> int step_cn2(ps3d_gpu_ctx *c, double *t, double dt)
         }
         op_cn2_update<T>(d, c->st, c->svor, c->vortsm, sv, c->filt0, c->fz, c->vdiss, dt2);
         op_mean_fix(d, c->st, c->svor, c->dstsum, c->fnzi, c->ini, nullptr, 1);
-        if (mixed) project_state_mixed(c);
+        if (mixed) project_state_mixed(c, true);
         c->launches += 4;
     }
     *t += dt;
@@ -1317,14 +1319,13 @@ __global__ void k_vdiss_dev(long long n, const double *vhdis, double *vdiss, con
 int dev_pre(ps3d_gpu_ctx *c)
 {
     const Dims &d = c->d;
-    const long long N = d.nfield;
     int rc = vor2vel<float>(c);
     if (rc) return rc;
     red_pass1<float>(d, c->st, tf<float>(c->vel), tf<float>(c->vor), c->part, c->res1);
     float *g5 = tmpf<float>(c, 0);
     op_strain_fields<float>(d, c->st, c->D(), tf<float>(c->svel), g5);
     c->launches += 3;
-    for (int k = 0; k < 5; ++k) xyi<float>(c, g5 + k * N, g5 + k * N);
+    xyi<float>(c, g5, g5, 5);
     cudaMemsetAsync(c->flag, 0, sizeof(int), c->st);
     red_pass2<float>(d, c->st, tf<float>(c->vor), g5, 0.0, c->part, c->res2, c->flag, nullptr, c->res1,
                      (double)c->ncell);
@@ -1926,7 +1927,7 @@ void host_tables(ps3d_gpu_ctx *c)
 template <typename T> void twiddles(ps3d_gpu_ctx *c, void *dst, int n, int len)
 {
     std::vector<CT<T>> tw(n);
-    if (sizeof(T) == sizeof(double) && fx_serves(len)) {
+    if (sizeof(T) == sizeof(double) && c->d.fx64 && fx_serves(len)) {
         fx_twiddles(tw.data(), n);
         cudaMemcpyAsync(dst, tw.data(), n * sizeof(CT<T>), cudaMemcpyHostToDevice, c->st);
         cudaStreamSynchronize(c->st);
@@ -2027,7 +2028,7 @@ template <typename T> int allocate_fields(ps3d_gpu_ctx *c)
              dalloc(c, &c->cosz32, d.nz * sizeof(float)) &&
              dalloc(c, &c->stage64, f64) && dalloc(c, &c->phim64, f64) && dalloc(c, &c->phip64, f64) &&
              dalloc(c, &c->twx64, d.nx * sizeof(double2)) && dalloc(c, &c->twy64, d.ny * sizeof(double2)) &&
-             dalloc(c, &c->twz2_64, 2 * d.nz * sizeof(double2));
+             dalloc(c, &c->twz2_64, 2 * d.nz * sizeof(double2)) && dalloc(c, &c->twz2_fx, 2 * d.nz * sizeof(double2));
     const size_t P2 = (size_t)d.ncol * sizeof(double), Z = (size_t)(d.nz + 1) * sizeof(double);
     ok = ok && dalloc(c, &c->twx, d.nx * sizeof(CT<T>)) && dalloc(c, &c->twy, d.ny * sizeof(CT<T>)) &&
          dalloc(c, &c->twz2, 2 * d.nz * sizeof(CT<T>));
@@ -2051,12 +2052,19 @@ template <typename T> int allocate_fields(ps3d_gpu_ctx *c)
         c->twx64 = tf<double2>(c->twx);
         c->twy64 = tf<double2>(c->twy);
         c->twz2_64 = tf<double2>(c->twz2);
+        c->twz2_fx = c->twz2;
         c->phim64 = tf<double>(c->phim);
         c->phip64 = tf<double>(c->phip);
     } else {
         twiddles<double>(c, c->twx64, d.nx, d.nx);
         twiddles<double>(c, c->twy64, d.ny, d.ny);
         twiddles<double>(c, c->twz2_64, 2 * d.nz, d.nz);
+        if (fx_serves(d.nz)) {
+            std::vector<double2> tw(2 * d.nz);
+            fx_twiddles(tw.data(), 2 * d.nz);
+            cudaMemcpyAsync(c->twz2_fx, tw.data(), tw.size() * sizeof(double2), cudaMemcpyHostToDevice, c->st);
+            cudaStreamSynchronize(c->st);
+        }
         twiddles<float>(c, c->twz32, d.nz, d.nz);
         std::vector<float> sn(d.nz), cs(d.nz);
         for (int j = 0; j < d.nz; ++j) {
@@ -2177,6 +2185,7 @@ int ps3d_gpu_create(const ps3d_gpu_config *cfg, ps3d_gpu_ctx **out)
     c->serial = ++next_serial;
     c->cfg = *cfg;
     c->fp64 = cfg->precision == PS3D_PRECISION_FP64;
+    c->d.fx64 = c->fp64;
     cudaSetDevice(cfg->device);
     transforms_init();
     columns32_init();

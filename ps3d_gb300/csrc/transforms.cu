@@ -112,7 +112,7 @@ int lines_lanes(int n)
 template <typename T>
 void launch_lines(cudaStream_t st, const T *in, T *out, int n, int P, int zv, long long line_stride,
                   long long nbatch, long long batch_stride, bool inverse,
-                  const typename cplx<T>::type *tw, int shape = -1, int nf = 1, long long fs_in = 0,
+                  const typename cplx<T>::type *tw, bool fx64, int shape = -1, int nf = 1, long long fs_in = 0,
                   long long fs_out = 0)
 {
     if constexpr (sizeof(T) == sizeof(float)) {
@@ -124,7 +124,7 @@ void launch_lines(cudaStream_t st, const T *in, T *out, int n, int P, int zv, lo
         }
     }
     if constexpr (sizeof(T) == sizeof(double)) {
-        if (fx_serves(n)) {
+        if (fx64 && fx_serves(n)) {
             fx_lines(st, reinterpret_cast<const double *>(in), reinterpret_cast<double *>(out), n, P, zv, line_stride,
                      nbatch, batch_stride, inverse, tw, nf, fs_in, fs_out);
             return;
@@ -158,7 +158,7 @@ void y_forward(const Dims &d, cudaStream_t st, const T *in, T *out, const typena
                int nf)
 {
     if (pr) pr->begin(PROBE_YLINES, st);
-    launch_lines<T>(st, in, out, d.ny, d.P, d.nz + 1, d.P, d.nx, (long long)d.ny * d.P, false, twy, d.line_shape[0],
+    launch_lines<T>(st, in, out, d.ny, d.P, d.nz + 1, d.P, d.nx, (long long)d.ny * d.P, false, twy, d.fx64, d.line_shape[0],
                     nf, d.nfield, d.nfield);
     if (pr) pr->end(PROBE_YLINES, st, nf * pass_bytes<T>(d));
 }
@@ -168,7 +168,7 @@ void x_forward(const Dims &d, cudaStream_t st, const T *in, T *out, const typena
                int nf)
 {
     if (pr) pr->begin(PROBE_XLINES, st);
-    launch_lines<T>(st, in, out, d.nx, d.P, d.nz + 1, (long long)d.ny * d.P, d.ny, d.P, false, twx, d.line_shape[1],
+    launch_lines<T>(st, in, out, d.nx, d.P, d.nz + 1, (long long)d.ny * d.P, d.ny, d.P, false, twx, d.fx64, d.line_shape[1],
                     nf, d.nfield, d.nfield);
     if (pr) pr->end(PROBE_XLINES, st, nf * pass_bytes<T>(d));
 }
@@ -178,7 +178,7 @@ void x_inverse(const Dims &d, cudaStream_t st, const T *in, T *out, const typena
                int nf)
 {
     if (pr) pr->begin(PROBE_XLINES, st);
-    launch_lines<T>(st, in, out, d.nx, d.P, d.nz + 1, (long long)d.ny * d.P, d.ny, d.P, true, twx, d.line_shape[3],
+    launch_lines<T>(st, in, out, d.nx, d.P, d.nz + 1, (long long)d.ny * d.P, d.ny, d.P, true, twx, d.fx64, d.line_shape[3],
                     nf, d.nfield, d.nfield);
     if (pr) pr->end(PROBE_XLINES, st, nf * pass_bytes<T>(d));
 }
@@ -188,7 +188,7 @@ void y_inverse(const Dims &d, cudaStream_t st, const T *in, T *out, const typena
                int nf)
 {
     if (pr) pr->begin(PROBE_YLINES, st);
-    launch_lines<T>(st, in, out, d.ny, d.P, d.nz + 1, d.P, d.nx, (long long)d.ny * d.P, true, twy, d.line_shape[2],
+    launch_lines<T>(st, in, out, d.ny, d.P, d.nz + 1, d.P, d.nx, (long long)d.ny * d.P, true, twy, d.fx64, d.line_shape[2],
                     nf, d.nfield, d.nfield);
     if (pr) pr->end(PROBE_YLINES, st, nf * pass_bytes<T>(d));
 }
@@ -331,7 +331,7 @@ void columns(const Dims &d, cudaStream_t st, int mode, const T *in, T *out, cons
              const T *phip, const typename cplx<T>::type *twz2, Probe *pr, int nf)
 {
     if constexpr (sizeof(T) == sizeof(double)) {
-        if (fx_serves(d.nz)) {
+        if (d.fx64 && fx_serves(d.nz)) {
             if (pr) pr->begin(PROBE_COLUMNS, st);
             fx_columns(d, st, mode, in, out, phim, phip, twz2, nf);
             if (pr) pr->end(PROBE_COLUMNS, st, nf * pass_bytes<T>(d));
