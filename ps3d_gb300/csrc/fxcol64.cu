@@ -436,11 +436,16 @@ __global__ void __launch_bounds__(256) k_fx_src(const double *__restrict__ f, do
 
 // levels per lane and pairs per block of a column length: 8 pairs (one warp
 // each) up to 128 levels, 4 pairs of two warps above (48 nz bytes of shared
-// memory per pair: four blocks per SM up to 256)
-template <typename F> static void col_shape(int nz, F f)
+// memory per pair: four blocks per SM up to 256) and where 8 pairs would make
+// fewer than two blocks per SM (32^3: w and dw/dz 18.7 us with 8 pairs, 17.0
+// with 4)
+template <typename F> static void col_shape(int nz, long long ncol, F f)
 {
     using std::integral_constant;
-    if (nz <= 64) f(integral_constant<int, 2>(), integral_constant<int, 3>());
+    const bool few = ncol < 2 * 152 * 16;
+    if (nz <= 64 && few) f(integral_constant<int, 1>(), integral_constant<int, 2>());
+    else if (nz <= 64) f(integral_constant<int, 2>(), integral_constant<int, 3>());
+    else if (nz <= 128 && few) f(integral_constant<int, 2>(), integral_constant<int, 2>());
     else if (nz <= 128) f(integral_constant<int, 4>(), integral_constant<int, 3>());
     else if (nz <= 256) f(integral_constant<int, 4>(), integral_constant<int, 2>());
     else f(integral_constant<int, 8>(), integral_constant<int, 2>());
@@ -455,7 +460,7 @@ void fx_columns(const Dims &d, cudaStream_t st, int mode, const double *in, doub
 {
     const Tw *W = reinterpret_cast<const Tw *>(tw);
     const fx::Plan pl = fx::col_plan(d.nz);
-    col_shape(d.nz, [&](auto nit, auto lb) {
+    col_shape(d.nz, d.ncol, [&](auto nit, auto lb) {
         constexpr int NIT = decltype(nit)::value, LB = decltype(lb)::value;
         const auto go = [&](auto kern) {
             kern<<<col_grid(d, LB, nf), 256, (size_t)d.nz * 48 << LB, st>>>(in, out, d.nz, d.P, d.ncol, d.nfield, phim,
@@ -471,7 +476,7 @@ void fx_comdec(const Dims &d, cudaStream_t st, const double *c, double *cs, doub
                const double *phim, const double *phip, const void *tw)
 {
     const fx::Plan pl = fx::col_plan(d.nz);
-    col_shape(d.nz, [&](auto nit, auto lb) {
+    col_shape(d.nz, d.ncol, [&](auto nit, auto lb) {
         constexpr int NIT = decltype(nit)::value, LB = decltype(lb)::value;
         k_fx_comdec<NIT, LB><<<col_grid(d, LB, 1), 256, (size_t)d.nz * 48 << LB, st>>>(
             c, cs, es, d.nz, d.P, d.ncol, dzi, phim, phip, pl, reinterpret_cast<const Tw *>(tw));
@@ -483,7 +488,7 @@ void fx_w(const Dims &d, cudaStream_t st, const double *A, const double *B, doub
 {
     const fx::Plan pl = fx::col_plan(d.nz);
     const WTables tb{thetam, thetap, dthetam, dthetap, green, rkz};
-    col_shape(d.nz, [&](auto nit, auto lb) {
+    col_shape(d.nz, d.ncol, [&](auto nit, auto lb) {
         constexpr int NIT = decltype(nit)::value, LB = decltype(lb)::value;
         k_fx_w<NIT, LB><<<col_grid(d, LB, 1), 256, (size_t)d.nz * 48 << LB, st>>>(
             A, B, w, es, d.nx, d.ny, d.nz, d.P, d.ncol, D, tb, pl, reinterpret_cast<const Tw *>(tw));
@@ -493,7 +498,7 @@ void fx_src(const Dims &d, cudaStream_t st, const double *f, double *out, const 
             const double *phip, const void *tw)
 {
     const fx::Plan pl = fx::col_plan(d.nz);
-    col_shape(d.nz, [&](auto nit, auto lb) {
+    col_shape(d.nz, d.ncol, [&](auto nit, auto lb) {
         constexpr int NIT = decltype(nit)::value, LB = decltype(lb)::value;
         k_fx_src<NIT, LB><<<col_grid(d, LB, 3), 256, (size_t)d.nz * 48 << LB, st>>>(
             f, out, d.nx, d.ny, d.nz, d.P, d.ncol, d.nfield, D, phim, phip, pl, reinterpret_cast<const Tw *>(tw));
@@ -502,8 +507,8 @@ void fx_src(const Dims &d, cudaStream_t st, const double *f, double *out, const 
 
 void fx_columns_init()
 {
-    for (int nz : {64, 128, 256, 512})
-        col_shape(nz, [&](auto nit, auto lb) {
+    for (int nz : {64, 128, 256, 512, -64, -128})
+        col_shape(nz < 0 ? -nz : nz, nz < 0 ? 0 : 1 << 20, [&](auto nit, auto lb) {
             constexpr int NIT = decltype(nit)::value, LB = decltype(lb)::value;
             const auto set = [](auto kern) {
                 cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
