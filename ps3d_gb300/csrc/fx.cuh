@@ -501,6 +501,65 @@ FX_FN I2 *passes(I2 *s, I2 *d, int n, int nseq, int ns, const Tw *__restrict__ t
     }
     return s;
 }
+// A pass in place: thread tid of nthreads reads and transforms all its
+// butterflies (at most ceil(R1 / R): there are n B / R1 threads), then, when
+// every thread has read, writes them.  nthreads is a multiple of B.
+template <int R1, int R, bool INV, int LB> struct PassRegs {
+    static constexpr int NB = (R1 + R - 1) / R, B = 1 << LB;
+    I2 v[NB][R];
+    int o[NB];
+    FX_FN void read(const I2 *buf, int n, int Ns, const Tw *__restrict__ tw, int tid, int nthreads)
+    {
+        const int nR = n / R, nbf = nR << LB, twstride = nR / Ns, b = tid & (B - 1);
+#pragma unroll
+        for (int q = 0; q < NB; ++q) {
+            const int h = tid + q * nthreads;
+            o[q] = -1;
+            if (h < nbf) {
+                const int j = h >> LB;
+                const int k = ((Ns & (Ns - 1)) == 0) ? (j & (Ns - 1)) : (j % Ns);
+#pragma unroll
+                for (int r = 0; r < R; ++r) v[q][r] = buf[at<LB>(j + r * nR, b)];
+                // a radix below 8: doubled first, so the product divides by 2
+                v[q][0] = up_shift(R) ? mk2((v[q][0].x + 1) >> 1, (v[q][0].y + 1) >> 1) : quarter(v[q][0]);
+                const Tw *t = tw;
+#pragma unroll
+                for (int r = 1; r < R; ++r) {
+                    t += k * twstride;
+                    if (up_shift(R)) v[q][r] = add(v[q][r], v[q][r]);
+                    v[q][r] = cmulw(v[q][r], *t, INV);
+                }
+                dft<R, INV>(v[q]);
+                o[q] = (j - k) * R + k;
+            }
+        }
+    }
+    FX_FN void write(I2 *buf, int Ns, int tid) const
+    {
+#pragma unroll
+        for (int q = 0; q < NB; ++q)
+            if (o[q] >= 0) {
+#pragma unroll
+                for (int r = 0; r < R; ++r) buf[at<LB>(o[q] + r * Ns, tid & (B - 1))] = v[q][r];
+            }
+    }
+};
+// the passes of a line after its first, of radix R1, in place; run(pass, Ns)
+// carries out one (pass: a PassRegs type's empty value)
+template <int R1, bool INV, int LB, typename RUN> FX_FN void later_passes(int n, RUN run)
+{
+    int Ns = R1;
+    for (int rem = n / R1; rem > 1;) {
+        const int r = next_radix(rem);
+        if (R1 == 8 && r == 8) run(PassRegs<R1, 8, INV, LB>(), Ns);
+        else if (R1 == 8 && r == 4) run(PassRegs<R1, 4, INV, LB>(), Ns);
+        else if (r == 2) run(PassRegs<R1, 2, INV, LB>(), Ns);
+        else if (r == 3) run(PassRegs<R1, 3, INV, LB>(), Ns);
+        else run(PassRegs<R1, 5, INV, LB>(), Ns);
+        Ns *= r;
+        rem /= r;
+    }
+}
 // the first pass from shared memory (column sequences)
 template <int R, bool INV, int LB>
 FX_FN void pass1(const I2 *src, I2 *dst, int n, int nseq, int tid, int nthreads)

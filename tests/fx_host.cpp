@@ -36,7 +36,7 @@ static void line(int n, int inverse, const double *a, const double *b, double *o
 {
     const Plan pl = line_plan(n, inverse != 0);
     const vector<Tw> tw = table(n);
-    vector<I2> b0((size_t)n << LB), b1(b0.size());
+    vector<I2> b0((size_t)n << LB);
     const unsigned ma = top(a, n), mb = top(b, n);
     const int ea = line_exp(ma), eb = line_exp(mb), h = n / 2;
     const int Ea = bits_of(a, n, ma, pl), Eb = bits_of(b, n, mb, pl);
@@ -51,9 +51,16 @@ static void line(int n, int inverse, const double *a, const double *b, double *o
             if (inverse) first_pass<R, true, LB>(v, b0.data(), j, p);
             else first_pass<R, false, LB>(v, b0.data(), j, p);
         }
-    auto nobar = [] {};
-    const I2 *q = inverse ? passes<true, LB>(b0.data(), b1.data(), n, 1, R, tw.data(), 1, 0, 1, nobar)
-                          : passes<false, LB>(b0.data(), b1.data(), n, 1, R, tw.data(), 1, 0, 1, nobar);
+    // the later passes in place, all threads of a block reading before any writes
+    const int nt = (((n / R) << LB) + 31) / 32 * 32;
+    const auto run = [&](auto pass, int Ns) {
+        vector<decltype(pass)> regs(nt);
+        for (int t = 0; t < nt; ++t) regs[t].read(b0.data(), n, Ns, tw.data(), t, nt);
+        for (int t = 0; t < nt; ++t) regs[t].write(b0.data(), Ns, t);
+    };
+    if (inverse) later_passes<R, true, LB>(n, run);
+    else later_passes<R, false, LB>(n, run);
+    const I2 *q = b0.data();
     const Scale sa = scale_of(ma, Ea, pl), sb = scale_of(mb, Eb, pl);
     const int p = (1 << LB) - 1;
     for (int k = 0; k < n; ++k) {
@@ -72,12 +79,12 @@ static void line(int n, int inverse, const double *a, const double *b, double *o
         }
     }
 }
-extern "C" void fx_line(int n, int inverse, int wide, const double *a, const double *b, double *oa, double *ob)
+extern "C" void fx_line(int n, int inverse, int, const double *a, const double *b, double *oa, double *ob)
 {
     const int r = first_radix(n);
-    if (r == 8) wide ? line<8, 3>(n, inverse, a, b, oa, ob) : line<8, 2>(n, inverse, a, b, oa, ob);
-    else if (r == 4) wide ? line<4, 3>(n, inverse, a, b, oa, ob) : line<4, 2>(n, inverse, a, b, oa, ob);
-    else if (r == 5) wide ? line<5, 3>(n, inverse, a, b, oa, ob) : line<5, 2>(n, inverse, a, b, oa, ob);
+    if (r == 8) line<8, 2>(n, inverse, a, b, oa, ob);
+    else if (r == 4) line<4, 2>(n, inverse, a, b, oa, ob);
+    else if (r == 5) line<5, 2>(n, inverse, a, b, oa, ob);
     else line<3, 1>(n, inverse, a, b, oa, ob);
 }
 

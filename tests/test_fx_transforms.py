@@ -111,7 +111,7 @@ def test_scales_and_non_finite_lines(host, scale):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("shape", [(8, 10, 8), (12, 30, 10), (60, 8, 288), (32, 32, 30), (128, 12, 72), (8, 512, 12),
-                                   (10, 24, 512)])
+                                   (10, 24, 512), (18, 250, 24), (500, 54, 8)])
 def test_operators_device(shape):
     """every tile tail: odd z counts, few pairs per block, ragged columns"""
     from ps3d_gb300 import Ps3dGpu
