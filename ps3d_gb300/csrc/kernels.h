@@ -200,6 +200,9 @@ void op_v2v_ds(const Dims &d, cudaStream_t st, const Deriv &D, const S *A, const
 template <typename T, typename S>
 void op_v2v_project(const Dims &d, cudaStream_t st, const Deriv &D, const double *k2l2i, const T *es,
                     const T *ds, S *A, S *B);
+// the same with ds = D_x B - D_y A formed inside, in place (FP64 form)
+void op_project64(const Dims &d, cudaStream_t st, const Deriv &D, const double *k2l2i, const double *es, double *A,
+                  double *B);
 template <typename T, typename S>
 void op_v2v_wsrc(const Dims &d, cudaStream_t st, const Deriv &D, const S *A, const S *B, T *ds);
 template <typename T>
@@ -233,15 +236,16 @@ template <typename T, typename S>
 void op_add(const Dims &d, cudaStream_t st, S *acc, const T *add, long long n);
 
 // steppers
+// ncomp components nfield apart per launch
 template <typename T>
-void op_rk4_sub1(const Dims &d, cudaStream_t st, double *q, double *qdi, double *qdf, T *sqs,
-                 const double *filt0, const double *emq, double dt2, double dt6);
+void op_rk4_sub1(const Dims &d, cudaStream_t st, double *q, double *qdi, double *qdf, const T *sqs,
+                 const double *filt0, const double *emq, double dt2, double dt6, int ncomp);
 template <typename T>
 void op_rk4_sub23(const Dims &d, cudaStream_t st, double *q, const double *qdi, double *qdf, const T *sqs,
-                  const double *epq, const double *emq, double c1, double dt3);
+                  const double *epq, const double *emq, double c1, double dt3, int ncomp);
 template <typename T>
 void op_rk4_sub4(const Dims &d, cudaStream_t st, double *q, const double *qdf, const T *sqs,
-                 const double *epq, const double *emq, double dt6);
+                 const double *epq, const double *emq, double dt6, int ncomp);
 void op_rk4_factors(const Dims &d, cudaStream_t st, const double *vdiss, const double *filt0, double *epq,
                     double *emq, double *epq2, double *emq2);
 template <typename T>

@@ -110,7 +110,10 @@ void op_v2v_wsrc(const Dims &d, cudaStream_t st, const Deriv &D, const S *A, con
 // another, so one block takes the whole orbit: e and f are read once instead
 // of twice.  Same expression per output as the per-column form.  MEAN: the
 // (0,0) column gets ubar, vbar; otherwise it is left as it is.
-template <typename T, typename S, bool MEAN>
+// FOLD: k2l2i folded into the derivative coefficients first (four FP64
+// operations per element instead of six; the FP64 form, whose pipe bounds it:
+// 256^3 213 us before, 151 folded).
+template <typename T, typename S, bool MEAN, bool FOLD = false>
 __global__ void __launch_bounds__(128) k_v2v_orbit(Dims d, Deriv D, const double *__restrict__ k2l2i,
                                                    const T *__restrict__ e, const T *__restrict__ f,
                                                    const double *__restrict__ ubar, const double *__restrict__ vbar,
@@ -138,7 +141,12 @@ __global__ void __launch_bounds__(128) k_v2v_orbit(Dims d, Deriv D, const double
             }
         return;  // the (0,0) orbit has no other member
     }
-    const S cx = (S)D.cx[mx], cy = (S)D.cy[my], kk = (S)k2l2i[col];
+    S cx = (S)D.cx[mx], cy = (S)D.cy[my];
+    const S kk = (S)k2l2i[col];
+    if (FOLD) {
+        cx *= kk;
+        cy *= kk;
+    }
     auto ld = [&](const T *g, int iz) { return (active && iz <= d.nz) ? (S)g[o + iz] : (S)0; };
     S ev = ld(e, lane), fv = ld(f, lane);
     int buf = 0;
@@ -152,8 +160,10 @@ __global__ void __launch_bounds__(128) k_v2v_orbit(Dims d, Deriv D, const double
         }
         __syncthreads();
         if (active && iz <= d.nz) {
-            a[o + iz] = kk * (cx * sh_e[buf][xw][lane] + cy * sh_f[buf][yw][lane]);
-            b[o + iz] = kk * (cy * sh_e[buf][yw][lane] - cx * sh_f[buf][xw][lane]);
+            const S p = cx * sh_e[buf][xw][lane] + cy * sh_f[buf][yw][lane];
+            const S q = cy * sh_e[buf][yw][lane] - cx * sh_f[buf][xw][lane];
+            a[o + iz] = FOLD ? p : kk * p;
+            b[o + iz] = FOLD ? q : kk * q;
         }
     }
 }
@@ -167,6 +177,55 @@ void op_v2v_project(const Dims &d, cudaStream_t st, const Deriv &D, const double
                     const T *ds, S *A, S *B)
 {
     k_v2v_orbit<T, S, false><<<orbit_blocks(d), 128, 0, st>>>(d, D, k2l2i, es, ds, nullptr, nullptr, A, B);
+}
+
+// The projection of the FP64 form's vor2vel with ds = D_x B - D_y A formed on
+// chip, in place: A = k2l2i (D_x es + D_y ds), B = k2l2i (D_y es - D_x ds) on
+// each partner orbit, k2l2i folded into the coefficients (six FP64 operations
+// per element instead of eight, and ds neither written nor read: 256^3 73 +
+// 213 us as two kernels, 220 us here).
+__global__ void __launch_bounds__(128) k_project_orbit(Dims d, Deriv D, const double *__restrict__ k2l2i,
+                                                       const double *__restrict__ es, double *A, double *B)
+{
+    __shared__ double sh_a[2][4][32], sh_b[2][4][32], sh_e[2][4][32], sh_d[2][4][32];
+    const int hy = d.ny / 2 + 1;
+    const long long orb = blockIdx.x;
+    const int kx = (int)(orb / hy), ky = (int)(orb - (long long)kx * hy);
+    const int x2 = xsrc(kx, d.nx), y2 = xsrc(ky, d.ny);
+    const bool dx = x2 != kx, dy = y2 != ky;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool active = (!(w & 1) || dx) && (!(w & 2) || dy);
+    const int mx = (w & 1) ? x2 : kx, my = (w & 2) ? y2 : ky;
+    const int xw = dx ? (w ^ 1) : w, yw = dy ? (w ^ 2) : w;
+    const long long col = (long long)my + (long long)d.ny * mx, o = col * d.P;
+    if (orb == 0) return;  // the (0,0) column keeps its mean vorticity
+    const double cx = D.cx[mx], cy = D.cy[my], kk = k2l2i[col], px = kk * cx, py = kk * cy;
+    auto ld = [&](const double *g, int iz) { return (active && iz <= d.nz) ? g[o + iz] : 0.0; };
+    double av = ld(A, lane), bv = ld(B, lane), ev = ld(es, lane);
+    int buf = 0;
+    for (int z0 = 0; z0 <= d.nz; z0 += 32, buf ^= 1) {
+        const int iz = z0 + lane;
+        sh_a[buf][w][lane] = av;
+        sh_b[buf][w][lane] = bv;
+        sh_e[buf][w][lane] = ev;
+        if (z0 + 32 <= d.nz) {
+            av = ld(A, iz + 32);
+            bv = ld(B, iz + 32);
+            ev = ld(es, iz + 32);
+        }
+        __syncthreads();
+        sh_d[buf][w][lane] = cx * sh_b[buf][xw][lane] - cy * sh_a[buf][yw][lane];
+        __syncthreads();
+        if (active && iz <= d.nz) {
+            A[o + iz] = px * sh_e[buf][xw][lane] + py * sh_d[buf][yw][lane];
+            B[o + iz] = py * sh_e[buf][yw][lane] - px * sh_d[buf][xw][lane];
+        }
+    }
+}
+void op_project64(const Dims &d, cudaStream_t st, const Deriv &D, const double *k2l2i, const double *es, double *A,
+                  double *B)
+{
+    k_project_orbit<<<orbit_blocks(d), 128, 0, st>>>(d, D, k2l2i, es, A, B);
 }
 
 // boundary contributions and Green-function inversion for w
@@ -270,7 +329,7 @@ template <typename T>
 void op_v2v_uv(const Dims &d, cudaStream_t st, const Deriv &D, const double *k2l2i, const T *es, const T *cs,
                const double *ubar, const double *vbar, T *u, T *v)
 {
-    k_v2v_orbit<T, T, true><<<orbit_blocks(d), 128, 0, st>>>(d, D, k2l2i, es, cs, ubar, vbar, u, v);
+    k_v2v_orbit<T, T, true, sizeof(T) == 8><<<orbit_blocks(d), 128, 0, st>>>(d, D, k2l2i, es, cs, ubar, vbar, u, v);
 }
 
 // ------------------------------------------------------------------- source
@@ -660,26 +719,26 @@ void op_rk4_factors(const Dims &d, cudaStream_t st, const double *vdiss, const d
 // substep 1 (impl_rk4.f90:212-242)
 template <typename T>
 __global__ void k_rk4_sub1(Dims d, double *__restrict__ q, double *__restrict__ qdi, double *__restrict__ qdf,
-                           T *__restrict__ sqs, const double *__restrict__ filt0, const double *__restrict__ emq,
+                           const T *__restrict__ sqs, const double *__restrict__ filt0, const double *__restrict__ emq,
                            double dt2, double dt6)
 {
     COLUMN_HEADER
+    const long long c = blockIdx.y * d.nfield;  // component
     const double f0 = filt0[col], m = emq[col];
     for (int iz = threadIdx.x; iz <= d.nz; iz += 32) {
-        const long long i = o + iz;
+        const long long i = c + o + iz;
         const double s = f0 * (double)sqs[i];
         const double q0 = q[i];
-        sqs[i] = (T)s;
         qdi[i] = q0;
         q[i] = (q0 + dt2 * s) * m;
         qdf[i] = q0 + dt6 * s;
     }
 }
 template <typename T>
-void op_rk4_sub1(const Dims &d, cudaStream_t st, double *q, double *qdi, double *qdf, T *sqs,
-                 const double *filt0, const double *emq, double dt2, double dt6)
+void op_rk4_sub1(const Dims &d, cudaStream_t st, double *q, double *qdi, double *qdf, const T *sqs,
+                 const double *filt0, const double *emq, double dt2, double dt6, int ncomp)
 {
-    k_rk4_sub1<T><<<col_grid(d), COL_BLOCK, 0, st>>>(d, q, qdi, qdf, sqs, filt0, emq, dt2, dt6);
+    k_rk4_sub1<T><<<dim3(col_grid(d).x, ncomp), COL_BLOCK, 0, st>>>(d, q, qdi, qdf, sqs, filt0, emq, dt2, dt6);
 }
 
 // substeps 2 and 3 (impl_rk4.f90:247-326): c1 = dt/2 or dt
@@ -689,9 +748,10 @@ __global__ void k_rk4_sub23(Dims d, double *__restrict__ q, const double *__rest
                             const double *__restrict__ emq, double c1, double dt3)
 {
     COLUMN_HEADER
+    const long long c = blockIdx.y * d.nfield;  // component
     const double pp = epq[col], m = emq[col];
     for (int iz = threadIdx.x; iz <= d.nz; iz += 32) {
-        const long long i = o + iz;
+        const long long i = c + o + iz;
         const double s = pp * (double)sqs[i];
         q[i] = (qdi[i] + c1 * s) * m;
         qdf[i] = qdf[i] + dt3 * s;
@@ -699,9 +759,9 @@ __global__ void k_rk4_sub23(Dims d, double *__restrict__ q, const double *__rest
 }
 template <typename T>
 void op_rk4_sub23(const Dims &d, cudaStream_t st, double *q, const double *qdi, double *qdf, const T *sqs,
-                  const double *epq, const double *emq, double c1, double dt3)
+                  const double *epq, const double *emq, double c1, double dt3, int ncomp)
 {
-    k_rk4_sub23<T><<<col_grid(d), COL_BLOCK, 0, st>>>(d, q, qdi, qdf, sqs, epq, emq, c1, dt3);
+    k_rk4_sub23<T><<<dim3(col_grid(d).x, ncomp), COL_BLOCK, 0, st>>>(d, q, qdi, qdf, sqs, epq, emq, c1, dt3);
 }
 
 // substep 4 (impl_rk4.f90:331-364)
@@ -711,17 +771,18 @@ __global__ void k_rk4_sub4(Dims d, double *__restrict__ q, const double *__restr
                            const double *__restrict__ emq, double dt6)
 {
     COLUMN_HEADER
+    const long long c = blockIdx.y * d.nfield;  // component
     const double pp = epq[col], m = emq[col];
     for (int iz = threadIdx.x; iz <= d.nz; iz += 32) {
-        const long long i = o + iz;
+        const long long i = c + o + iz;
         q[i] = (qdf[i] + dt6 * (pp * (double)sqs[i])) * m;
     }
 }
 template <typename T>
 void op_rk4_sub4(const Dims &d, cudaStream_t st, double *q, const double *qdf, const T *sqs,
-                 const double *epq, const double *emq, double dt6)
+                 const double *epq, const double *emq, double dt6, int ncomp)
 {
-    k_rk4_sub4<T><<<col_grid(d), COL_BLOCK, 0, st>>>(d, q, qdf, sqs, epq, emq, dt6);
+    k_rk4_sub4<T><<<dim3(col_grid(d).x, ncomp), COL_BLOCK, 0, st>>>(d, q, qdf, sqs, epq, emq, dt6);
 }
 
 // Mixed form: the increment (c1 * epq * sqs, an FP32 source term scaled by
@@ -1910,12 +1971,12 @@ void op_hyperbolic_tables(const Dims &d, cudaStream_t st, const double *k2l2, co
                                const T *, const T *, T *, T *, T *);                                           \
     template void op_strain_fields<T>(const Dims &, cudaStream_t, const Deriv &, const T *, T *);              \
     template void op_add<T, double>(const Dims &, cudaStream_t, double *, const T *, long long);              \
-    template void op_rk4_sub1<T>(const Dims &, cudaStream_t, double *, double *, double *, T *,               \
-                                 const double *, const double *, double, double);                              \
+    template void op_rk4_sub1<T>(const Dims &, cudaStream_t, double *, double *, double *, const T *,         \
+                                 const double *, const double *, double, double, int);                         \
     template void op_rk4_sub23<T>(const Dims &, cudaStream_t, double *, const double *, double *, const T *,  \
-                                  const double *, const double *, double, double);                             \
+                                  const double *, const double *, double, double, int);                        \
     template void op_rk4_sub4<T>(const Dims &, cudaStream_t, double *, const double *, const T *,             \
-                                 const double *, const double *, double);                                      \
+                                 const double *, const double *, double, int);                                 \
     template void op_cn2_init<T>(const Dims &, cudaStream_t, double *, const double *, const T *, double, int); \
     template void op_cn2_update<T>(const Dims &, cudaStream_t, double *, const double *, const T *,           \
                                    const double *, const double *, const double *, double, int);               \

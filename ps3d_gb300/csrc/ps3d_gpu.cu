@@ -459,10 +459,9 @@ int vor2vel_fp64(ps3d_gpu_ctx *c)
     const Deriv D = c->D();
 
     // solenoidal projection (inversion.f90:34-76)
-    op_v2v_ds<T, double>(d, c->st, D, A, B, ds);
     combine_diffz64(c, Cc, cs, es, true);
-    op_v2v_project<T, double>(d, c->st, D, c->k2l2i, es, ds, A, B);
-    c->launches += 2;
+    op_project64(d, c->st, D, c->k2l2i, es, A, B);
+    c->launches += 1;
 
     // vorticity in physical space (field_combine_physical x3, :80-82): the
     // first two components combined straight into vor, x lines of those in
@@ -1058,7 +1057,7 @@ template <typename T> int step_rk4(ps3d_gpu_ctx *c, double *t, double dt)
         if (mixed)
             op_rk4m_sub1(d, c->st, c->sbuoy, c->sbuoyi, accb, sb32, c->sbuoy32, c->filt0, c->bmq, dtp);
         else
-            op_rk4_sub1<T>(d, c->st, c->sbuoy, c->sbuoyi, c->sbuoyf, sb, c->filt0, c->bmq, dt2, dt6);
+            op_rk4_sub1<T>(d, c->st, c->sbuoy, c->sbuoyi, c->sbuoyf, sb, c->filt0, c->bmq, dt2, dt6, 1);
         c->launches += 1;
     }
     // the mixed form: projection, filter and stage update in one pass per
@@ -1076,10 +1075,8 @@ template <typename T> int step_rk4(ps3d_gpu_ctx *c, double *t, double dt)
     if (mixed) {
         stage(1, c->filt0, c->emq);
     } else {
-        for (int k = 0; k < 3; ++k)
-            op_rk4_sub1<T>(d, c->st, c->svor + k * N, c->svori + k * N, c->svorf + k * N, sv + k * N, c->filt0,
-                           c->emq, dt2, dt6);
-        c->launches += 3;
+        op_rk4_sub1<T>(d, c->st, c->svor, c->svori, c->svorf, sv, c->filt0, c->emq, dt2, dt6, 3);
+        c->launches += 1;
     }
     int rc = rhs_or_hold<T>(c);
     if (rc) return rc;
@@ -1088,16 +1085,14 @@ template <typename T> int step_rk4(ps3d_gpu_ctx *c, double *t, double dt)
         if (mixed)
             op_rk4m_sub23(d, c->st, c->sbuoy, c->sbuoyi, accb, sb32, c->sbuoy32, c->bpq, c->bmq, dtp, false);
         else
-            op_rk4_sub23<T>(d, c->st, c->sbuoy, c->sbuoyi, c->sbuoyf, sb, c->bpq, c->bmq, dt2, dt3);
+            op_rk4_sub23<T>(d, c->st, c->sbuoy, c->sbuoyi, c->sbuoyf, sb, c->bpq, c->bmq, dt2, dt3, 1);
         c->launches += 1;
     }
     if (mixed) {
         stage(2, c->epq, c->emq);
     } else {
-        for (int k = 0; k < 3; ++k)
-            op_rk4_sub23<T>(d, c->st, c->svor + k * N, c->svori + k * N, c->svorf + k * N, sv + k * N, c->epq,
-                            c->emq, dt2, dt3);
-        c->launches += 3;
+        op_rk4_sub23<T>(d, c->st, c->svor, c->svori, c->svorf, sv, c->epq, c->emq, dt2, dt3, 3);
+        c->launches += 1;
     }
     rc = rhs_or_hold<T>(c);
     if (rc) return rc;
@@ -1106,16 +1101,14 @@ template <typename T> int step_rk4(ps3d_gpu_ctx *c, double *t, double dt)
         if (mixed)
             op_rk4m_sub23(d, c->st, c->sbuoy, c->sbuoyi, accb, sb32, c->sbuoy32, c->bpq, c->bmq2, dtp, true);
         else
-            op_rk4_sub23<T>(d, c->st, c->sbuoy, c->sbuoyi, c->sbuoyf, sb, c->bpq, c->bmq2, dt, dt3);
+            op_rk4_sub23<T>(d, c->st, c->sbuoy, c->sbuoyi, c->sbuoyf, sb, c->bpq, c->bmq2, dt, dt3, 1);
         c->launches += 1;
     }
     if (mixed) {
         stage(3, c->epq, c->emq2);
     } else {
-        for (int k = 0; k < 3; ++k)
-            op_rk4_sub23<T>(d, c->st, c->svor + k * N, c->svori + k * N, c->svorf + k * N, sv + k * N, c->epq,
-                            c->emq2, dt, dt3);
-        c->launches += 3;
+        op_rk4_sub23<T>(d, c->st, c->svor, c->svori, c->svorf, sv, c->epq, c->emq2, dt, dt3, 3);
+        c->launches += 1;
     }
     rc = rhs_or_hold<T>(c);
     if (rc) return rc;
@@ -1123,15 +1116,14 @@ template <typename T> int step_rk4(ps3d_gpu_ctx *c, double *t, double dt)
         if (mixed)
             op_rk4m_sub4(d, c->st, c->sbuoy, c->sbuoyi, accb, sb32, c->sbuoy32, c->bpq2, c->bmq2, dtp);
         else
-            op_rk4_sub4<T>(d, c->st, c->sbuoy, c->sbuoyf, sb, c->bpq2, c->bmq2, dt6);
+            op_rk4_sub4<T>(d, c->st, c->sbuoy, c->sbuoyf, sb, c->bpq2, c->bmq2, dt6, 1);
         c->launches += 1;
     }
     if (mixed) {
         stage(4, c->epq2, c->emq2);
     } else {
-        for (int k = 0; k < 3; ++k)
-            op_rk4_sub4<T>(d, c->st, c->svor + k * N, c->svorf + k * N, sv + k * N, c->epq2, c->emq2, dt6);
-        c->launches += 3;
+        op_rk4_sub4<T>(d, c->st, c->svor, c->svorf, sv, c->epq2, c->emq2, dt6, 3);
+        c->launches += 1;
     }
     op_mean_fix(d, c->st, c->svor, c->dstsum, c->fnzi, c->ini, nullptr, 1, c->svor32);
     c->launches += 1;
