@@ -32,12 +32,16 @@ constexpr int PAIRS = 8;   // threads per row (two lanes each)
 // autotuner picks one per pass; by default the forward transform takes 0
 // and the inverse (its Hermitian first pass needs more registers) takes 1.
 // N = 1024 always runs one 512-thread block per SM (128 KB of shared
-// memory), N <= 256 three 256-thread blocks.
+// memory), N = 256 three 256-thread blocks.  A radix-8 pass has N / 8
+// butterflies for G = T / 8 groups, so N = 128 and 64 take 128 and 64 threads
+// (six and twelve blocks per SM): with 256 half and three quarters of the
+// warps had none (captured 128^3 step 1.243 ms with
+// 256 threads, 1.138 with 128; batch of twelve runs 85.6 and 78.6).
 template <int N, bool INV, int W> struct LinePlan {
     static constexpr bool BIG = N >= 1024 || (N == 512 && W == 0);
-    static constexpr int T = BIG ? 512 : 256;  // threads per block
-    static constexpr int G = T / PAIRS;        // butterfly groups
-    static constexpr int MINB = N >= 1024 ? 1 : (BIG ? 2 : 3);
+    static constexpr int T = BIG ? 512 : N >= 256 ? 256 : N;  // threads per block
+    static constexpr int G = T / PAIRS;                       // butterfly groups
+    static constexpr int MINB = N >= 1024 ? 1 : BIG ? 2 : 3 * 256 / T;
 };
 
 __device__ __forceinline__ float2 cm(float2 a, float2 b)
@@ -128,7 +132,9 @@ __device__ __forceinline__ void pass(float4 *sm, const float4 *__restrict__ gin,
 // 32 floats is 4 x 8 levels, 32 bytes of each.  Blocks are numbered z-tile
 // fastest, the tail blocks last.  5 tiles per batch become 4.25 at 128
 // levels: captured 128^3 step 1.271 -> 1.256 ms, batch of twelve runs
-// 88.5 -> 85.9 ms; at 512 levels 17 become 16.25, within the noise.
+// 88.5 -> 85.9 ms; 256^3 step 6.84 -> 6.77.  Above 264 levels the tail stays a
+// tile of its batch: at 512^3 the gain of 17 -> 16.25 tiles is lost again by
+// reading those 32-byte pieces apart from their rows (host step 72.4 -> 73.2).
 struct Tile {
     int z0;           // first level
     long long batch;  // (first) batch
@@ -142,7 +148,10 @@ struct Tile {
 struct Tiling {
     int full;          // 32-level tiles per batch
     long long nbatch;
-    __host__ __device__ static bool short_tail(int zv) { return zv % 32 >= 1 && zv % 32 <= 8 && zv > 32; }
+        __host__ __device__ static bool short_tail(int zv)
+    {
+        return zv % 32 >= 1 && zv % 32 <= 8 && zv > 32 && zv <= 8 * 32 + 8;
+    }
     static Tiling of(int zv, long long nbatch) { return Tiling{short_tail(zv) ? zv / 32 : (zv + 31) / 32, nbatch}; }
     unsigned blocks(int zv) const
     {
@@ -358,9 +367,8 @@ __global__ void __launch_bounds__(LinePlan<N, false, W>::T, LinePlan<N, false, W
     extern __shared__ __align__(16) float4 smL[];
     constexpr int T = LinePlan<N, false, W>::T, G = LinePlan<N, false, W>::G;
     constexpr int R = 8, NB = N / R, NBT = (NB + G - 1) / G;
-    // butterflies j >= NB (N <= 128) leave whole warps idle: a warp's four
-    // row groups are g = 4w..4w+3 and NB is a multiple of 4, so the
-    // shuffles below always run on full warps
+    // a warp's four row groups are g = 4w..4w+3 and NB is a multiple of 4, so
+    // the shuffles below always run on full warps
     static_assert(NB % 4 == 0 && PAIRS == 8, "warp-uniform butterfly ranges");
     const int o = blockIdx.x % 3;
     const Tile t = tiling.tile(blockIdx.x / 3);
