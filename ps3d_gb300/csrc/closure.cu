@@ -467,9 +467,23 @@ __global__ void __launch_bounds__(256) k_wgrad_reduce(const float *__restrict__ 
 // channel COUTP/4*(j/2) + 2n + j%2.  transpose != 0 builds the backward-data
 // image: input channels of the image = the layer's outputs, outputs = the
 // layer's inputs, taps mirrored.
-__global__ void k_wimage(const float *__restrict__ W, const float *__restrict__ b, int cin, int cout, int CINP,
-                         int COUTP, int transpose, uint2 *__restrict__ img, float *__restrict__ bpad)
+// One launch makes all of them (image blockIdx.y).
+struct WImage {
+    const float *W, *b;
+    int cin, cout, CINP, COUTP, transpose;
+    uint2 *img;
+    float *bpad;
+};
+struct WImages {
+    WImage i[2 * NL - 1];
+};
+__global__ void k_wimages(const __grid_constant__ WImages all)
 {
+    const WImage &a = all.i[blockIdx.y];
+    const float *W = a.W, *b = a.b;
+    const int cin = a.cin, cout = a.cout, CINP = a.CINP, COUTP = a.COUTP, transpose = a.transpose;
+    uint2 *img = a.img;
+    float *bpad = a.bpad;
     const int S = CINP / 16, NT = COUTP / 8;
     const int total = NTAP * S * NT * 32;
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1315,26 +1329,28 @@ void backward(ps3d_closure *cl, cudaStream_t st)
 }
 
 // rebuild the BF16 images from the FP32 master parameters
-void images(ps3d_closure *cl, cudaStream_t st)
+// tc: also the images of the tcgen05 inference engine
+void images(ps3d_closure *cl, cudaStream_t st, bool tc = true)
 {
-    for (int l = 0; l < NL; ++l) {
+    WImages w;
+    int n = 0, most = 0;
+    const auto put = [&](int l, int cinp, int coutp, int transpose, uint2 *img, float *bpad) {
         const float *W = cl->w + woff(l);
-        const float *b = W + NTAP * CREAL_IN[l] * CREAL_OUT[l];
-        const int nf = NTAP * (CPAD_IN[l] / 16) * (CPAD_OUT[l] / 8) * 32;
-        k_wimage<<<(nf + 255) / 256, 256, 0, st>>>(W, b, CREAL_IN[l], CREAL_OUT[l], CPAD_IN[l], CPAD_OUT[l], 0,
-                                                  cl->imgf[l], cl->bpad[l]);
-        if (l > 0) {
-            const int cinp = l == NL - 1 ? CPAD_DZ4 : CPAD_OUT[l];
-            const int nb = NTAP * (cinp / 16) * (CPAD_IN[l] / 8) * 32;
-            k_wimage<<<(nb + 255) / 256, 256, 0, st>>>(W, b, CREAL_IN[l], CREAL_OUT[l], cinp, CPAD_IN[l], 1,
-                                                      cl->imgb[l], nullptr);
-        }
-        if (cl->tc_ok) {
-            const int coutp = l == NL - 1 ? 16 : CPAD_OUT[l];
-            const int nt = NTAP * (CPAD_IN[l] / 8) * coutp;
-            k_wimage_tc<<<(nt + 255) / 256, 256, 0, st>>>(W, CREAL_IN[l], CREAL_OUT[l], CPAD_IN[l], coutp,
-                                                         cl->imgtc[l]);
-        }
+        w.i[n++] = WImage{W, W + NTAP * CREAL_IN[l] * CREAL_OUT[l], CREAL_IN[l], CREAL_OUT[l], cinp, coutp, transpose,
+                          img, bpad};
+        const int e = NTAP * (cinp / 16) * (coutp / 8) * 32;
+        most = e > most ? e : most;
+    };
+    for (int l = 0; l < NL; ++l) {
+        put(l, CPAD_IN[l], CPAD_OUT[l], 0, cl->imgf[l], cl->bpad[l]);
+        if (l > 0) put(l, l == NL - 1 ? CPAD_DZ4 : CPAD_OUT[l], CPAD_IN[l], 1, cl->imgb[l], nullptr);
+    }
+    k_wimages<<<dim3((most + 255) / 256, n), 256, 0, st>>>(w);
+    for (int l = 0; l < NL && tc && cl->tc_ok; ++l) {
+        const int coutp = l == NL - 1 ? 16 : CPAD_OUT[l];
+        const int nt = NTAP * (CPAD_IN[l] / 8) * coutp;
+        k_wimage_tc<<<(nt + 255) / 256, 256, 0, st>>>(cl->w + woff(l), CREAL_IN[l], CREAL_OUT[l], CPAD_IN[l], coutp,
+                                                     cl->imgtc[l]);
     }
 }
 
@@ -1679,7 +1695,7 @@ int ps3d_closure_train(ps3d_closure *cl, int iters, double lr0, double lr1, unsi
         const float c2 = (float)(1.0 / (1.0 - std::pow((double)b2, (double)cl->adam_t)));
         k_adam<<<(NPARAM + 255) / 256, 256, 0, cl->st>>>(cl->w, cl->g, cl->m, cl->v, NPARAM, (float)lr, b1, b2, c1, c2,
                                                          1e-8f);
-        images(cl, cl->st);
+        images(cl, cl->st, it + 1 == iters);  // the steps use the warp engine's images
         if ((it & 63) == 63) {
             rc = ccheck(cl, "train");
             if (rc) return rc;
