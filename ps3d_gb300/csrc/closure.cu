@@ -671,23 +671,24 @@ __global__ void k_adam(float *__restrict__ w, const float *__restrict__ g, float
 // ===================================================== tcgen05 inference path
 // The forward pass on the 5th-generation tensor cores.  Activations live in a
 // padded, channel-chunk-planar layout: padded row r = GUARD + (iz+1) +
-// ZP*((iy+1) + YP*(ix+1)) (ZP = nz+3, YP = ny+2), chunk plane kc (8 channels,
+// ZP*((iy+1) + YP*(ix+1)) (ZP = nz+3 rounded up to 8, YP = ny+2), chunk plane kc (8 channels,
 // 16 bytes) at byte (kc*RTOT + r)*16.  Ghost rows at iz = -1, nz+1 stay zero
-// (the z zero padding); ghost rows at iy = -1, ny and ix = -1, nx hold the
+// (the z zero padding, and what rounds ZP up); ghost rows at iy = -1, ny and ix = -1, nx hold the
 // periodic copies, written by the producer of each activation; GUARD rows
 // before and after keep every load of a tile in bounds.  Every tap is then a
-// uniform shift of the row index, so one tile of 128 output rows needs, per x
-// shift dx, one contiguous run of 128 + 2(ZP+1) rows per chunk plane: 3 x KC
-// one-dimensional TMA bulk copies.  The 27 taps x CIN/16 k-steps are
-// tcgen05.mma (M 128, N = COUT, K 16, BF16 in, FP32 accumulate in TMEM)
-// issued by one thread from shared-memory descriptors shifted by
-// (ZP*dy + dz) rows (no-swizzle K-major core matrices: 8 rows x 16 bytes,
-// SBO 128 bytes between row groups, LBO one chunk plane); the epilogue reads
-// the accumulator with tcgen05.ld (one TMEM lane per thread = one output row).
+// uniform shift of the row index, so one tile of 128 rows needs, per x shift
+// dx, one contiguous run of 128 + 2 ZP rows per chunk plane: 3 x KC
+// one-dimensional TMA bulk copies.  The 9 neighbour columns x CIN/16 k-steps
+// are tcgen05.mma (M 128, N = 3 COUT for the three dz taps, K 16, BF16 in,
+// FP32 accumulate in TMEM) issued by one thread from shared-memory
+// descriptors shifted by ZP*dy rows (no-swizzle K-major core matrices: 8 rows
+// x 16 bytes, SBO 128 bytes between row groups, LBO one chunk plane); the
+// epilogue reads the accumulators with tcgen05.ld (one TMEM lane per thread =
+// one row) and adds the three taps of an output row.
 
 struct TcArgs {
     const unsigned char *in;   // padded chunk-planar input (CIN/8 planes)
-    const uint4 *wimg;         // [tap][kc][co] x 16 bytes
+    const uint4 *wimg;         // [dx dy][kc][dz][co] x 16 bytes
     const float *bias;         // [COUT]
     unsigned char *out;        // EPI_GELU: padded chunk-planar activation
     float *outf;               // EPI_OUT: [npts][CPAD_OUT] FP32
@@ -708,11 +709,11 @@ __device__ __forceinline__ uint64_t tc_desc(uint32_t saddr, uint32_t lbo, uint32
     return d;
 }
 
-template <int COUT> __host__ __device__ constexpr uint32_t tc_idesc()
+template <int N> __host__ __device__ constexpr uint32_t tc_idesc()
 {
     // kind::f16: D F32 (bits 4-5 = 1), A BF16 (7-9 = 1), B BF16 (10-12 = 1),
     // both K-major, N >> 3 at 17-22, M >> 4 at 24-28 (M = 128)
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(COUT >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 }
 
 __device__ __forceinline__ void mbar_init(uint32_t a, uint32_t count)
@@ -831,14 +832,14 @@ __global__ void k_pack_pad(const T *__restrict__ vor, const T *__restrict__ vel,
     }
 }
 
-// [tap][kc][co] x 8 BF16 weight image of one layer for the tcgen05 kernel
+// [dx dy][kc][dz][co] x 8 BF16 weight image of one layer for the tcgen05 kernel
 __global__ void k_wimage_tc(const float *__restrict__ W, int cin, int cout, int CINP, int COUTP, uint4 *__restrict__ img)
 {
     const int KC = CINP / 8;
     const int total = NTAP * KC * COUTP;
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= total) return;
-    const int co = e % COUTP, kc = (e / COUTP) % KC, tap = e / (COUTP * KC);
+    const int co = e % COUTP, dz = (e / COUTP) % 3, kc = (e / (3 * COUTP)) % KC, tap = e / (3 * COUTP * KC) * 3 + dz;
     float w[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
@@ -849,7 +850,7 @@ __global__ void k_wimage_tc(const float *__restrict__ W, int cin, int cout, int 
 }
 
 template <int CIN, int COUT> __host__ __device__ constexpr int tc_wbytes() { return NTAP * (CIN / 8) * COUT * 16; }
-__host__ __device__ inline int tc_seg(int ZP) { return 128 + 2 * (ZP + 1); }
+__host__ __device__ inline int tc_seg(int ZP) { return 128 + 2 * ZP; }
 // weights + two tile buffers of 3 x CIN/8 chunk planes
 template <int CIN, int COUT> __host__ __device__ inline size_t tc_smem(int ZP)
 {
@@ -897,26 +898,39 @@ __device__ __forceinline__ void mbar_arrive(uint32_t a)
 }
 
 // One convolution layer over the padded grid, warp-specialised.  Persistent
-// CTAs of 9 warps walk tiles of 128 padded rows.  Warp 8 (one elected lane)
-// is the producer and issuer: TMA copies of tile k+1 into the shared buffer
-// freed by the products of tile k-1, and the 27 x CIN/16 tcgen05.mma of tile
-// k into TMEM accumulator k%2 once the epilogue has released it.  Warps 0-7
-// are the epilogue: they wait for the products of tile k, read their lane
-// quarter (warp % 4) and column half (warp / 4) of the accumulator, release
-// it, and apply bias + GELU and the stores.  The roles meet only on
-// mbarriers: full[b] (copies landed), done[b] (products complete, tcgen05.
-// commit), free[b] (256 epilogue arrivals).  Every wait is bounded; a wait
-// that runs out sets a shared flag that stops both roles, raises the error
-// word, and the issuer lets its operations in flight finish (bounded) before
-// the accumulator is released.
+// CTAs of 9 warps walk tiles of 128 padded rows, 126 of them outputs.  The
+// three dz taps of a neighbour column (dx, dy) are one product of N = 3 COUT:
+// D_dz(r) = sum over (dx, dy) of W_dz X(r), and the epilogue adds
+// D_-1(r - 1) + D_0(r) + D_+1(r + 1).  An operand row block is then read from
+// shared memory 9 times instead of 27, always from a multiple of 8 rows (ZP
+// is one): with 27 products of N = COUT that began at any row, shared-memory
+// reads of the rows bounded the layer (64^3: 32 -> 32 channels 60 us,
+// 16 -> 32 37, 32 -> 8 51; here @TC1, @TC2, @TC3).
+//
+// Warp 8 (one elected lane) is the producer and issuer: TMA copies of tile
+// k+1 into the shared buffer freed by the products of tile k-1, and the
+// 9 x CIN/16 tcgen05.mma of tile k into TMEM accumulator k%2 once the
+// epilogue has released it.  Warps 0-7 are the epilogue: they wait for the
+// products of tile k, read their lane quarter (warp % 4) and column half
+// (warp / 4) of the three accumulators, release them, exchange the rows next
+// to a quarter's edge through shared memory, and apply bias + GELU and the
+// stores.  The roles meet only on mbarriers: full[b] (copies landed), done[b]
+// (products complete, tcgen05.commit), free[b] (256 epilogue arrivals), and
+// edge[b][half] (the four warps of a column half have put their edge rows).
+// Every wait is bounded; a wait that runs out sets a shared flag that stops
+// both roles, raises the error word, and the issuer lets its operations in
+// flight finish (bounded) before the accumulator is released.
+constexpr int TC_ROWS = 126;  // outputs per tile
 template <int CIN, int COUT, int EPI>
 __global__ void __launch_bounds__(288, 1) k_conv_tc(TcArgs a)
 {
     constexpr int KC = CIN / 8, S = CIN / 16;
     constexpr int WB = tc_wbytes<CIN, COUT>();
-    constexpr uint32_t IDESC = tc_idesc<COUT>();
+    constexpr int N3 = 3 * COUT, H = COUT / 2;
+    constexpr uint32_t IDESC = tc_idesc<N3>();
     extern __shared__ __align__(1024) unsigned char smem[];
-    __shared__ __align__(8) uint64_t mbar[6];  // full[0..1], done[2..3], free[4..5]
+    __shared__ __align__(8) uint64_t mbar[10];  // full[0..1], done[2..3], free[4..5], edge[6 + 2 b + half]
+    __shared__ float edge[2][2][4][2][H];       // [b][half][quarter][last row of D_-1, first row of D_+1]
     __shared__ uint32_t tmem_slot;
     __shared__ volatile int bad;
     __shared__ float sbias[32];
@@ -933,11 +947,12 @@ __global__ void __launch_bounds__(288, 1) k_conv_tc(TcArgs a)
         for (int i = 0; i < 4; ++i) mbar_init(smem_u32(&mbar[i]), 1);
         mbar_init(smem_u32(&mbar[4]), 256);
         mbar_init(smem_u32(&mbar[5]), 256);
+        for (int i = 6; i < 10; ++i) mbar_init(smem_u32(&mbar[i]), 4);
         bad = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
     if (warp == 8) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 64;\n" ::"r"(smem_u32(&tmem_slot))
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 256;\n" ::"r"(smem_u32(&tmem_slot))
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
@@ -947,14 +962,15 @@ __global__ void __launch_bounds__(288, 1) k_conv_tc(TcArgs a)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
-    const long long ntiles = (a.QN + 127) / 128;
+    const long long ntiles = (a.QN + TC_ROWS - 1) / TC_ROWS;
     const long long nk = ntiles > (long long)blockIdx.x ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-    auto tile_q0 = [&](long long k) { return ((long long)blockIdx.x + k * (long long)gridDim.x) * 128; };
+    // first row of tile k: the one before its first output
+    auto tile_q0 = [&](long long k) { return ((long long)blockIdx.x + k * (long long)gridDim.x) * TC_ROWS - 1; };
 
     if (warp == 8) {
         if (lane == 0) {
             const uint32_t sAu = smem_u32(sA), sWu = smem_u32(sW);
-            const uint64_t bd0 = tc_desc(sWu, COUT * 16u, 128u);
+            const uint64_t bd0 = tc_desc(sWu, N3 * 16u, 128u);
             const int seg = (int)(segb >> 4);
             // phase parities and pending operations as bit masks (bit i:
             // barrier i; pending bits 0-3: copies into buffer 0/1, products
@@ -976,7 +992,7 @@ __global__ void __launch_bounds__(288, 1) k_conv_tc(TcArgs a)
                 mbar_expect_tx(mb, abuf);
                 const long long q0 = tile_q0(k);
                 for (int dxi = 0; dxi < 3; ++dxi) {
-                    const long long r0 = a.GUARD + q0 + (dxi - 1) * plane - (ZP + 1);
+                    const long long r0 = a.GUARD + q0 + (dxi - 1) * plane - ZP;
                     for (int kc = 0; kc < KC; ++kc)
                         bulk_g2s(sAu + (uint32_t)b * abuf + (uint32_t)(dxi * KC + kc) * segb,
                                  a.in + ((long long)kc * a.RTOT + r0) * 16, segb, mb);
@@ -988,7 +1004,7 @@ __global__ void __launch_bounds__(288, 1) k_conv_tc(TcArgs a)
                 if (!wait_bar(b)) break;                          // tile k in shared memory
                 if (k >= 2 && !wait_bar(4 + b)) break;            // epilogue of tile k-2 released accumulator b
                 tc_fence_after();
-                const uint32_t acc = tmem + (uint32_t)(b * 32);
+                const uint32_t acc = tmem + (uint32_t)(b * 128);
                 // descriptors = base descriptor + start offset in 16-byte units
                 // (the 14-bit start field cannot carry below 256 KB)
                 const uint64_t ad0 = tc_desc(sAu + (uint32_t)b * abuf, segb, 128u);
@@ -997,16 +1013,14 @@ __global__ void __launch_bounds__(288, 1) k_conv_tc(TcArgs a)
 #pragma unroll
                     for (int dyi = 0; dyi < 3; ++dyi)
 #pragma unroll
-                        for (int dzi = 0; dzi < 3; ++dzi)
-#pragma unroll
-                            for (int s2 = 0; s2 < S; ++s2) {
-                                const int tap = dxi * 9 + dyi * 3 + dzi;
-                                // row offset of the tap in the tile buffer, >= 0
-                                const int off = (dxi * KC + 2 * s2) * seg + (ZP + 1) + ZP * (dyi - 1) + (dzi - 1);
-                                const uint64_t ad = ad0 + (uint64_t)(uint32_t)off;
-                                const uint64_t bd = bd0 + (uint64_t)((tap * KC + 2 * s2) * COUT);
-                                tc_mma(acc, ad, bd, IDESC, (tap | s2) != 0 ? 1u : 0u);
-                            }
+                        for (int s2 = 0; s2 < S; ++s2) {
+                            const int dxy = dxi * 3 + dyi;
+                            // row offset of the neighbour column in the tile buffer
+                            const int off = (dxi * KC + 2 * s2) * seg + ZP * dyi;
+                            const uint64_t ad = ad0 + (uint64_t)(uint32_t)off;
+                            const uint64_t bd = bd0 + (uint64_t)((dxy * KC + 2 * s2) * N3);
+                            tc_mma(acc, ad, bd, IDESC, (dxy | s2) != 0 ? 1u : 0u);
+                        }
                 pend |= 1u << (2 + b);
                 tc_commit(smem_u32(&mbar[2 + b]));
                 if (k + 1 < nk) {
@@ -1027,7 +1041,7 @@ __global__ void __launch_bounds__(288, 1) k_conv_tc(TcArgs a)
         }
     } else {
         const int quarter = warp & 3, half = warp >> 2;
-        uint32_t ph_done = 0u;  // bit b: phase parity of done[b]
+        uint32_t ph_done = 0u, ph_edge = 0u;  // bit b: phase parity of done[b], edge[b][half]
         for (long long k = 0; k < nk; ++k) {
             // warp-uniform decisions: the TMEM load below is warp-collective
             if (__any_sync(0xffffffffu, bad != 0)) break;
@@ -1039,19 +1053,50 @@ __global__ void __launch_bounds__(288, 1) k_conv_tc(TcArgs a)
             }
             ph_done ^= 1u << b;
             tc_fence_after();
-            float v[16];
-            const uint32_t taddr = tmem + (uint32_t)(b * 32 + half * (COUT / 2)) + ((uint32_t)(quarter * 32) << 16);
-            if (COUT == 32) tc_ld16(taddr, v);
-            else tc_ld8(taddr, v);
+            float v[16], m[16], p[16];  // D_0, D_-1, D_+1
+            const uint32_t taddr = tmem + (uint32_t)(b * 128 + half * H) + ((uint32_t)(quarter * 32) << 16);
+            if (COUT == 32) {
+                tc_ld16(taddr, m);
+                tc_ld16(taddr + COUT, v);
+                tc_ld16(taddr + 2 * COUT, p);
+            } else {
+                tc_ld8(taddr, m);
+                tc_ld8(taddr + COUT, v);
+                tc_ld8(taddr + 2 * COUT, p);
+            }
             tc_fence_before();
             mbar_arrive(smem_u32(&mbar[4 + b]));  // accumulator b may take the products of tile k+2
-            tc_epilogue<COUT, EPI>(a, sbias, (unsigned)(tile_q0(k) + quarter * 32 + lane), half, v);
+            if (lane == 31) {
+#pragma unroll
+                for (int j = 0; j < H; ++j) edge[b][half][quarter][0][j] = m[j];
+            }
+            if (lane == 0) {
+#pragma unroll
+                for (int j = 0; j < H; ++j) edge[b][half][quarter][1][j] = p[j];
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&mbar[6 + 2 * b + half]));
+            const bool met = mbar_wait(smem_u32(&mbar[6 + 2 * b + half]), (ph_edge >> b) & 1u);
+            if (!__all_sync(0xffffffffu, met)) {
+                bad = 1;
+                break;
+            }
+            ph_edge ^= 1u << b;
+#pragma unroll
+            for (int j = 0; j < H; ++j) {
+                float below = __shfl_up_sync(0xffffffffu, m[j], 1), above = __shfl_down_sync(0xffffffffu, p[j], 1);
+                if (lane == 0 && quarter > 0) below = edge[b][half][quarter - 1][0][j];
+                if (lane == 31 && quarter < 3) above = edge[b][half][quarter + 1][1][j];
+                v[j] = (below + v[j]) + above;
+            }
+            const int row = quarter * 32 + lane;
+            if (row > 0 && row <= TC_ROWS) tc_epilogue<COUT, EPI>(a, sbias, (unsigned)(tile_q0(k) + row), half, v);
         }
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (warp == 8) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 64;\n" ::"r"(tmem) : "memory");
+    if (warp == 8) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;\n" ::"r"(tmem) : "memory");
 }
 
 // host-side SplitMix64 (parameter initialisation, sample order)
@@ -1209,13 +1254,13 @@ template <int CIN, int COUT, int EPI> bool tc_attr(ps3d_closure *cl)
         cudaGetLastError();
         return false;
     }
-    cl->tc_occ[tc_slot<CIN, COUT, EPI>()] = nb;
+    cl->tc_occ[tc_slot<CIN, COUT, EPI>()] = nb < 2 ? nb : 2;  // 256 of an SM's 512 TMEM columns each
     return true;
 }
 
 template <int CIN, int COUT, int EPI> void conv_tc(ps3d_closure *cl, cudaStream_t st, const TcArgs &a)
 {
-    const long long ntiles = (cl->QN + 127) / 128;
+    const long long ntiles = (cl->QN + TC_ROWS - 1) / TC_ROWS;
     const long long maxb = (long long)cl->nsm * cl->tc_occ[tc_slot<CIN, COUT, EPI>()];
     const long long per = (ntiles + maxb - 1) / maxb;
     const unsigned grid = (unsigned)((ntiles + per - 1) / per);
@@ -1486,13 +1531,15 @@ int ps3d_closure_create(int nx, int ny, int nz, int max_samples, int device, uns
     cudaFuncSetAttribute(k_wgrad<32, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * WG<32, 32>::BUF);
     cudaFuncSetAttribute(k_wgrad<32, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * WG<32, 16>::BUF);
     // tcgen05 path: padded geometry; available when a tile's shared memory
-    // (weights + 3 x 4 chunk planes of 128 + 2(ZP+1) rows) fits a block
-    cl->ZP = nz + 3;
+    // (weights + 3 x 4 chunk planes of 128 + 2 ZP rows) fits a block
+    // z pitch of a padded column: a multiple of 8 where a tile then still fits
+    cl->ZP = (nz + 3 + 7) / 8 * 8;
+    if (tc_smem<32, 32>(cl->ZP) + 4096 > (size_t)prop.sharedMemPerBlockOptin) cl->ZP = nz + 3;
     cl->YP = ny + 2;
     cl->QN = (long long)(nx + 2) * cl->YP * cl->ZP;
     cl->GUARD = (long long)cl->YP * cl->ZP + cl->ZP + 256;
     cl->RTOT = (cl->QN + 2 * cl->GUARD + 7) / 8 * 8;
-    cl->tc_ok = tc_smem<32, 32>(cl->ZP) + 2048 <= (size_t)prop.sharedMemPerBlockOptin && tc_attr<16, 32, EPI_GELU>(cl) &&
+    cl->tc_ok = tc_smem<32, 32>(cl->ZP) + 4096 <= (size_t)prop.sharedMemPerBlockOptin && tc_attr<16, 32, EPI_GELU>(cl) &&
                 tc_attr<32, 32, EPI_GELU>(cl) && tc_attr<32, 16, EPI_OUT>(cl);
     cl->engine = cl->tc_ok ? PS3D_CLOSURE_ENGINE_TCGEN05 : PS3D_CLOSURE_ENGINE_MMA;
     const long long P = cl->npts;
