@@ -694,6 +694,7 @@ struct TcArgs {
     float *outf;               // EPI_OUT: [npts][CPAD_OUT] FP32
     int *err;                  // device error word (bounded waits)
     int nx, ny, Z, ZP, YP;
+    int nbuf;                  // tile buffers (2..4)
     long long QN, RTOT, GUARD, npts;
 };
 
@@ -851,11 +852,12 @@ __global__ void k_wimage_tc(const float *__restrict__ W, int cin, int cout, int 
 
 template <int CIN, int COUT> __host__ __device__ constexpr int tc_wbytes() { return NTAP * (CIN / 8) * COUT * 16; }
 __host__ __device__ inline int tc_seg(int ZP) { return 128 + 2 * ZP; }
-// weights + two tile buffers of 3 x CIN/8 chunk planes
-template <int CIN, int COUT> __host__ __device__ inline size_t tc_smem(int ZP)
+// weights + nbuf tile buffers of 3 x CIN/8 chunk planes
+template <int CIN, int COUT> __host__ __device__ inline size_t tc_smem(int ZP, int nbuf = 2)
 {
-    return (size_t)tc_wbytes<CIN, COUT>() + (size_t)2 * 3 * (CIN / 8) * tc_seg(ZP) * 16;
+    return (size_t)tc_wbytes<CIN, COUT>() + (size_t)nbuf * 3 * (CIN / 8) * tc_seg(ZP) * 16;
 }
+constexpr size_t TC_STATIC = 7168;  // static shared memory and the block's share of the driver's
 
 // epilogue of one tile for one output row and one half of the accumulator
 // columns (v: COUT/2 values from column half*COUT/2): bias + GELU into the
@@ -898,21 +900,25 @@ __device__ __forceinline__ void mbar_arrive(uint32_t a)
 }
 
 // One convolution layer over the padded grid, warp-specialised.  Persistent
-// CTAs of 9 warps walk tiles of 128 padded rows, 126 of them outputs.  The
+// CTAs of 17 warps walk tiles of 128 padded rows, 126 of them outputs.  The
 // three dz taps of a neighbour column (dx, dy) are one product of N = 3 COUT:
 // D_dz(r) = sum over (dx, dy) of W_dz X(r), and the epilogue adds
 // D_-1(r - 1) + D_0(r) + D_+1(r + 1).  An operand row block is then read from
 // shared memory 9 times instead of 27, always from a multiple of 8 rows (ZP
 // is one): with 27 products of N = COUT that began at any row, shared-memory
 // reads of the rows bounded the layer (64^3: 32 -> 32 channels 60 us,
-// 16 -> 32 37, 32 -> 8 51; here @TC1, @TC2, @TC3).
+// 16 -> 32 37, 32 -> 8 51; as one product, with two buffers and eight epilogue
+// warps, 44, 36 and 38; with three or four buffers and sixteen, 41, 32 and 32).
 //
-// Warp 8 (one elected lane) is the producer and issuer: TMA copies of tile
-// k+1 into the shared buffer freed by the products of tile k-1, and the
+// Warp 16 (one elected lane) is the producer and issuer: TMA copies of tile
+// k-1+nbuf into the shared buffer freed by the products of tile k-1 (two
+// buffers left the copies' latency exposed; three or four where they fit), and
+// the
 // 9 x CIN/16 tcgen05.mma of tile k into TMEM accumulator k%2 once the
-// epilogue has released it.  Warps 0-7 are the epilogue: they wait for the
-// products of tile k, read their lane quarter (warp % 4) and column half
-// (warp / 4) of the three accumulators, release them, exchange the rows next
+// epilogue has released it.  Warps 0-15 are the epilogue, eight for the even
+// tiles and eight for the odd ones: they wait for the products of tile k, read
+// their lane quarter (warp % 4) and column half (warp / 4 % 2) of the three
+// accumulators, release them, exchange the rows next
 // to a quarter's edge through shared memory, and apply bias + GELU and the
 // stores.  The roles meet only on mbarriers: full[b] (copies landed), done[b]
 // (products complete, tcgen05.commit), free[b] (256 epilogue arrivals), and
@@ -921,16 +927,20 @@ __device__ __forceinline__ void mbar_arrive(uint32_t a)
 // both roles, raises the error word, and the issuer lets its operations in
 // flight finish (bounded) before the accumulator is released.
 constexpr int TC_ROWS = 126;  // outputs per tile
+constexpr int TC_ISSUER = 16, TC_THREADS = 32 * (TC_ISSUER + 1);
 template <int CIN, int COUT, int EPI>
-__global__ void __launch_bounds__(288, 1) k_conv_tc(TcArgs a)
+__global__ void __launch_bounds__(TC_THREADS, 1) k_conv_tc(TcArgs a)
 {
     constexpr int KC = CIN / 8, S = CIN / 16;
     constexpr int WB = tc_wbytes<CIN, COUT>();
     constexpr int N3 = 3 * COUT, H = COUT / 2;
     constexpr uint32_t IDESC = tc_idesc<N3>();
     extern __shared__ __align__(1024) unsigned char smem[];
-    __shared__ __align__(8) uint64_t mbar[10];  // full[0..1], done[2..3], free[4..5], edge[6 + 2 b + half]
-    __shared__ float edge[2][2][4][2][H];       // [b][half][quarter][last row of D_-1, first row of D_+1]
+    // full[0..3], done[4 + b], free[6 + b], edge[8 + 2 b + half]
+    __shared__ __align__(8) uint64_t mbar[12];
+    // [b][k / 2 % 2][half][quarter][last row of D_-1, first row of D_+1]: a warp
+    // two tiles ahead of its neighbour does not write what that one still reads
+    __shared__ float edge[2][2][2][4][2][H];
     __shared__ uint32_t tmem_slot;
     __shared__ volatile int bad;
     __shared__ float sbias[32];
@@ -944,19 +954,19 @@ __global__ void __launch_bounds__(288, 1) k_conv_tc(TcArgs a)
 
     if (tid < 32) sbias[tid] = tid < COUT ? a.bias[tid] : 0.f;
     if (tid == 0) {
-        for (int i = 0; i < 4; ++i) mbar_init(smem_u32(&mbar[i]), 1);
-        mbar_init(smem_u32(&mbar[4]), 256);
-        mbar_init(smem_u32(&mbar[5]), 256);
-        for (int i = 6; i < 10; ++i) mbar_init(smem_u32(&mbar[i]), 4);
+        for (int i = 0; i < 6; ++i) mbar_init(smem_u32(&mbar[i]), 1);
+        mbar_init(smem_u32(&mbar[6]), 256);
+        mbar_init(smem_u32(&mbar[7]), 256);
+        for (int i = 8; i < 12; ++i) mbar_init(smem_u32(&mbar[i]), 4);
         bad = 0;
         asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     }
-    if (warp == 8) {
+    if (warp == TC_ISSUER) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 256;\n" ::"r"(smem_u32(&tmem_slot))
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
-    for (int i = tid; i < WB / 16; i += 288) reinterpret_cast<uint4 *>(sW)[i] = __ldg(a.wimg + i);
+    for (int i = tid; i < WB / 16; i += TC_THREADS) reinterpret_cast<uint4 *>(sW)[i] = __ldg(a.wimg + i);
     asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     tc_fence_before();
     __syncthreads();
@@ -967,13 +977,13 @@ __global__ void __launch_bounds__(288, 1) k_conv_tc(TcArgs a)
     // first row of tile k: the one before its first output
     auto tile_q0 = [&](long long k) { return ((long long)blockIdx.x + k * (long long)gridDim.x) * TC_ROWS - 1; };
 
-    if (warp == 8) {
+    if (warp == TC_ISSUER) {
         if (lane == 0) {
             const uint32_t sAu = smem_u32(sA), sWu = smem_u32(sW);
             const uint64_t bd0 = tc_desc(sWu, N3 * 16u, 128u);
             const int seg = (int)(segb >> 4);
             // phase parities and pending operations as bit masks (bit i:
-            // barrier i; pending bits 0-3: copies into buffer 0/1, products
+            // barrier i; pending bits 0-3: copies into a buffer, 4-5: products
             // into accumulator 0/1), kept in registers
             uint32_t ph = 0u, pend = 0u;
             auto wait_bar = [&](int i) {
@@ -985,8 +995,8 @@ __global__ void __launch_bounds__(288, 1) k_conv_tc(TcArgs a)
                 bad = 1;
                 return false;
             };
-            auto issue_load = [&](long long k) {
-                const int b = (int)(k & 1);
+            const int nb = a.nbuf;
+            auto issue_load = [&](long long k, int b) {
                 const uint32_t mb = smem_u32(&mbar[b]);
                 pend |= 1u << b;
                 mbar_expect_tx(mb, abuf);
@@ -998,16 +1008,17 @@ __global__ void __launch_bounds__(288, 1) k_conv_tc(TcArgs a)
                                  a.in + ((long long)kc * a.RTOT + r0) * 16, segb, mb);
                 }
             };
-            if (nk > 0) issue_load(0);
+            for (int k = 0; k < nb - 1 && k < nk; ++k) issue_load(k, k);
+            int buf = 0;  // tile k's buffer
             for (long long k = 0; k < nk && !bad; ++k) {
                 const int b = (int)(k & 1);
-                if (!wait_bar(b)) break;                          // tile k in shared memory
-                if (k >= 2 && !wait_bar(4 + b)) break;            // epilogue of tile k-2 released accumulator b
+                if (!wait_bar(buf)) break;                        // tile k in shared memory
+                if (k >= 2 && !wait_bar(6 + b)) break;            // epilogue of tile k-2 released accumulator b
                 tc_fence_after();
                 const uint32_t acc = tmem + (uint32_t)(b * 128);
                 // descriptors = base descriptor + start offset in 16-byte units
                 // (the 14-bit start field cannot carry below 256 KB)
-                const uint64_t ad0 = tc_desc(sAu + (uint32_t)b * abuf, segb, 128u);
+                const uint64_t ad0 = tc_desc(sAu + (uint32_t)buf * abuf, segb, 128u);
 #pragma unroll
                 for (int dxi = 0; dxi < 3; ++dxi)
 #pragma unroll
@@ -1021,37 +1032,35 @@ __global__ void __launch_bounds__(288, 1) k_conv_tc(TcArgs a)
                             const uint64_t bd = bd0 + (uint64_t)((dxy * KC + 2 * s2) * N3);
                             tc_mma(acc, ad, bd, IDESC, (dxy | s2) != 0 ? 1u : 0u);
                         }
-                pend |= 1u << (2 + b);
-                tc_commit(smem_u32(&mbar[2 + b]));
-                if (k + 1 < nk) {
-                    // buffer 1-b is free once the products of tile k-1 are complete
-                    if (k >= 1 && !wait_bar(2 + (1 - b))) break;
-                    issue_load(k + 1);
-                }
+                pend |= 1u << (4 + b);
+                tc_commit(smem_u32(&mbar[4 + b]));
+                // the buffer of tile k-1 is free once its products are complete
+                if (k >= 1 && !wait_bar(4 + (1 - b))) break;
+                const int prev = buf == 0 ? nb - 1 : buf - 1;
+                if (k - 1 + nb < nk) issue_load(k - 1 + nb, prev);
+                buf = buf + 1 == nb ? 0 : buf + 1;
             }
             if (bad) {
                 atomicOr(a.err, 1);
-                for (int i = 0; i < 4; ++i)
+                for (int i = 0; i < 6; ++i)
                     if ((pend >> i) & 1u) mbar_wait(smem_u32(&mbar[i]), (ph >> i) & 1u);
             } else if (nk > 0) {
                 // the last tile's products (the epilogue waits for them too)
                 const int b = (int)((nk - 1) & 1);
-                if ((pend >> (2 + b)) & 1u) wait_bar(2 + b);
+                if ((pend >> (4 + b)) & 1u) wait_bar(4 + b);
             }
         }
     } else {
-        const int quarter = warp & 3, half = warp >> 2;
-        uint32_t ph_done = 0u, ph_edge = 0u;  // bit b: phase parity of done[b], edge[b][half]
-        for (long long k = 0; k < nk; ++k) {
+        const int quarter = warp & 3, half = (warp >> 2) & 1, b = warp >> 3;
+        uint32_t ph = 0u;  // phase parity of done[b] and edge[b][half]
+        for (long long k = b; k < nk; k += 2, ph ^= 1u) {
             // warp-uniform decisions: the TMEM load below is warp-collective
             if (__any_sync(0xffffffffu, bad != 0)) break;
-            const int b = (int)(k & 1);
-            const bool ok = mbar_wait(smem_u32(&mbar[2 + b]), (ph_done >> b) & 1u);
+            const bool ok = mbar_wait(smem_u32(&mbar[4 + b]), ph);
             if (!__all_sync(0xffffffffu, ok)) {
                 bad = 1;
                 break;
             }
-            ph_done ^= 1u << b;
             tc_fence_after();
             float v[16], m[16], p[16];  // D_0, D_-1, D_+1
             const uint32_t taddr = tmem + (uint32_t)(b * 128 + half * H) + ((uint32_t)(quarter * 32) << 16);
@@ -1065,28 +1074,28 @@ __global__ void __launch_bounds__(288, 1) k_conv_tc(TcArgs a)
                 tc_ld8(taddr + 2 * COUT, p);
             }
             tc_fence_before();
-            mbar_arrive(smem_u32(&mbar[4 + b]));  // accumulator b may take the products of tile k+2
+            mbar_arrive(smem_u32(&mbar[6 + b]));  // accumulator b may take the products of tile k+2
+            float(*eg)[2][H] = edge[b][(k >> 1) & 1][half];
             if (lane == 31) {
 #pragma unroll
-                for (int j = 0; j < H; ++j) edge[b][half][quarter][0][j] = m[j];
+                for (int j = 0; j < H; ++j) eg[quarter][0][j] = m[j];
             }
             if (lane == 0) {
 #pragma unroll
-                for (int j = 0; j < H; ++j) edge[b][half][quarter][1][j] = p[j];
+                for (int j = 0; j < H; ++j) eg[quarter][1][j] = p[j];
             }
             __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&mbar[6 + 2 * b + half]));
-            const bool met = mbar_wait(smem_u32(&mbar[6 + 2 * b + half]), (ph_edge >> b) & 1u);
+            if (lane == 0) mbar_arrive(smem_u32(&mbar[8 + 2 * b + half]));
+            const bool met = mbar_wait(smem_u32(&mbar[8 + 2 * b + half]), ph);
             if (!__all_sync(0xffffffffu, met)) {
                 bad = 1;
                 break;
             }
-            ph_edge ^= 1u << b;
 #pragma unroll
             for (int j = 0; j < H; ++j) {
                 float below = __shfl_up_sync(0xffffffffu, m[j], 1), above = __shfl_down_sync(0xffffffffu, p[j], 1);
-                if (lane == 0 && quarter > 0) below = edge[b][half][quarter - 1][0][j];
-                if (lane == 31 && quarter < 3) above = edge[b][half][quarter + 1][1][j];
+                if (lane == 0 && quarter > 0) below = eg[quarter - 1][0][j];
+                if (lane == 31 && quarter < 3) above = eg[quarter + 1][1][j];
                 v[j] = (below + v[j]) + above;
             }
             const int row = quarter * 32 + lane;
@@ -1096,7 +1105,7 @@ __global__ void __launch_bounds__(288, 1) k_conv_tc(TcArgs a)
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (warp == 8) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;\n" ::"r"(tmem) : "memory");
+    if (warp == TC_ISSUER) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;\n" ::"r"(tmem) : "memory");
 }
 
 // host-side SplitMix64 (parameter initialisation, sample order)
@@ -1133,7 +1142,8 @@ struct ps3d_closure {
     double *ctd = nullptr;   // ct in device memory; lpart[RED_BLOCKS]: one loss value
     // tcgen05 inference path: padded chunk-planar activations (input, two
     // ping-pong hidden buffers), weight images, device error word
-    int engine = 0, tc_ok = 0, tc_occ[3] = {1, 1, 1};
+    int engine = 0, tc_ok = 0, tc_occ[3] = {1, 1, 1}, tc_nbuf[3] = {2, 2, 2};
+    int smem_optin = 0;
     int ZP = 0, YP = 0;
     long long QN = 0, RTOT = 0, GUARD = 0;
     unsigned char *pa0 = nullptr, *pact[2] = {};
@@ -1242,14 +1252,18 @@ template <int CIN, int COUT, int EPI> constexpr int tc_slot() { return EPI == EP
 
 template <int CIN, int COUT, int EPI> bool tc_attr(ps3d_closure *cl)
 {
-    const size_t sm = tc_smem<CIN, COUT>(cl->ZP);
+    // as many buffers (to 4) as one block per SM can have
+    int nbuf = 2;
+    while (nbuf < 4 && tc_smem<CIN, COUT>(cl->ZP, nbuf + 1) + TC_STATIC <= (size_t)cl->smem_optin) ++nbuf;
+    const size_t sm = tc_smem<CIN, COUT>(cl->ZP, nbuf);
+    cl->tc_nbuf[tc_slot<CIN, COUT, EPI>()] = nbuf;
     if (cudaFuncSetAttribute(k_conv_tc<CIN, COUT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) !=
         cudaSuccess) {
         cudaGetLastError();
         return false;
     }
     int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_conv_tc<CIN, COUT, EPI>, 288, sm) != cudaSuccess ||
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_conv_tc<CIN, COUT, EPI>, TC_THREADS, sm) != cudaSuccess ||
         nb < 1) {
         cudaGetLastError();
         return false;
@@ -1264,7 +1278,9 @@ template <int CIN, int COUT, int EPI> void conv_tc(ps3d_closure *cl, cudaStream_
     const long long maxb = (long long)cl->nsm * cl->tc_occ[tc_slot<CIN, COUT, EPI>()];
     const long long per = (ntiles + maxb - 1) / maxb;
     const unsigned grid = (unsigned)((ntiles + per - 1) / per);
-    k_conv_tc<CIN, COUT, EPI><<<grid, 288, tc_smem<CIN, COUT>(cl->ZP), st>>>(a);
+    TcArgs b = a;
+    b.nbuf = cl->tc_nbuf[tc_slot<CIN, COUT, EPI>()];
+    k_conv_tc<CIN, COUT, EPI><<<grid, TC_THREADS, tc_smem<CIN, COUT>(cl->ZP, b.nbuf), st>>>(b);
 }
 
 // tcgen05 forward pass: pa0 -> pact[0] -> pact[1] -> pact[0] -> outf
@@ -1517,6 +1533,7 @@ int ps3d_closure_create(int nx, int ny, int nz, int max_samples, int device, uns
     cl->npts = (long long)nx * ny * (nz + 1);
     cl->device = device;
     cl->nsm = prop.multiProcessorCount;
+    cl->smem_optin = (int)prop.sharedMemPerBlockOptin;
     cl->max_samples = max_samples;
     cl->nchunk = (cl->npts + WG_CHUNK - 1) / WG_CHUNK;
     cl->rng.s = seed;
@@ -1534,12 +1551,12 @@ int ps3d_closure_create(int nx, int ny, int nz, int max_samples, int device, uns
     // (weights + 3 x 4 chunk planes of 128 + 2 ZP rows) fits a block
     // z pitch of a padded column: a multiple of 8 where a tile then still fits
     cl->ZP = (nz + 3 + 7) / 8 * 8;
-    if (tc_smem<32, 32>(cl->ZP) + 4096 > (size_t)prop.sharedMemPerBlockOptin) cl->ZP = nz + 3;
+    if (tc_smem<32, 32>(cl->ZP) + TC_STATIC > (size_t)prop.sharedMemPerBlockOptin) cl->ZP = nz + 3;
     cl->YP = ny + 2;
     cl->QN = (long long)(nx + 2) * cl->YP * cl->ZP;
     cl->GUARD = (long long)cl->YP * cl->ZP + cl->ZP + 256;
     cl->RTOT = (cl->QN + 2 * cl->GUARD + 7) / 8 * 8;
-    cl->tc_ok = tc_smem<32, 32>(cl->ZP) + 4096 <= (size_t)prop.sharedMemPerBlockOptin && tc_attr<16, 32, EPI_GELU>(cl) &&
+    cl->tc_ok = tc_smem<32, 32>(cl->ZP) + TC_STATIC <= (size_t)prop.sharedMemPerBlockOptin && tc_attr<16, 32, EPI_GELU>(cl) &&
                 tc_attr<32, 32, EPI_GELU>(cl) && tc_attr<32, 16, EPI_OUT>(cl);
     cl->engine = cl->tc_ok ? PS3D_CLOSURE_ENGINE_TCGEN05 : PS3D_CLOSURE_ENGINE_MMA;
     const long long P = cl->npts;
