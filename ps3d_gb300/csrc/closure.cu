@@ -857,7 +857,7 @@ template <int CIN, int COUT> __host__ __device__ inline size_t tc_smem(int ZP, i
 {
     return (size_t)tc_wbytes<CIN, COUT>() + (size_t)nbuf * 3 * (CIN / 8) * tc_seg(ZP) * 16;
 }
-constexpr size_t TC_STATIC = 7168;  // static shared memory and the block's share of the driver's
+constexpr size_t TC_STATIC = 2816;  // static shared memory of the kernel, rounded up
 
 // epilogue of one tile for one output row and one half of the accumulator
 // columns (v: COUT/2 values from column half*COUT/2): bias + GELU into the
@@ -935,12 +935,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_conv_tc(TcArgs a)
     constexpr int WB = tc_wbytes<CIN, COUT>();
     constexpr int N3 = 3 * COUT, H = COUT / 2;
     constexpr uint32_t IDESC = tc_idesc<N3>();
-    extern __shared__ __align__(1024) unsigned char smem[];
+    extern __shared__ __align__(128) unsigned char smem[];
     // full[0..3], done[4 + b], free[6 + b], edge[8 + 2 b + half]
     __shared__ __align__(8) uint64_t mbar[12];
-    // [b][k / 2 % 2][half][quarter][last row of D_-1, first row of D_+1]: a warp
-    // two tiles ahead of its neighbour does not write what that one still reads
-    __shared__ float edge[2][2][2][4][2][H];
+    // [b][half][quarter][last row of D_-1, first row of D_+1]; free[b] is arrived
+    // at after they are read, so the products of tile k+2, and with them the
+    // edge rows of tile k+2, come after every warp's reads
+    __shared__ float edge[2][2][4][2][H];
     __shared__ uint32_t tmem_slot;
     __shared__ volatile int bad;
     __shared__ float sbias[32];
@@ -1074,8 +1075,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_conv_tc(TcArgs a)
                 tc_ld8(taddr + 2 * COUT, p);
             }
             tc_fence_before();
-            mbar_arrive(smem_u32(&mbar[6 + b]));  // accumulator b may take the products of tile k+2
-            float(*eg)[2][H] = edge[b][(k >> 1) & 1][half];
+            float(*eg)[2][H] = edge[b][half];
             if (lane == 31) {
 #pragma unroll
                 for (int j = 0; j < H; ++j) eg[quarter][0][j] = m[j];
@@ -1098,6 +1098,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_conv_tc(TcArgs a)
                 if (lane == 31 && quarter < 3) above = eg[quarter + 1][1][j];
                 v[j] = (below + v[j]) + above;
             }
+            mbar_arrive(smem_u32(&mbar[6 + b]));  // accumulator b may take the products of tile k+2
             const int row = quarter * 32 + lane;
             if (row > 0 && row <= TC_ROWS) tc_epilogue<COUT, EPI>(a, sbias, (unsigned)(tile_q0(k) + row), half, v);
         }
