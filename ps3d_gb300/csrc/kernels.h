@@ -219,8 +219,6 @@ void op_v2v_uv(const Dims &d, cudaStream_t st, const Deriv &D, const double *k2l
                const double *ubar, const double *vbar, T *u, T *v);
 template <typename T>
 void op_add_const(const Dims &d, cudaStream_t st, T *f, double c);
-template <typename T>
-void op_products(const Dims &d, cudaStream_t st, const T *vel, const T *vor, T *r, T *q, T *p);
 // products and the z derivatives gq = dq/dz, gp = dp/dz in one pass
 template <typename T>
 void op_products_dz(const Dims &d, cudaStream_t st, double dzi, const T *vel, const T *vor, T *r, T *q, T *p,

@@ -345,36 +345,15 @@ template <typename T> void op_add_const(const Dims &d, cudaStream_t st, T *f, do
     k_add_const<T><<<col_grid(d), COL_BLOCK, 0, st>>>(d, f, c);
 }
 
-// r = u eta - v xi, q = w xi - u zeta, p = v zeta - w eta (inversion.f90:327-352)
-template <typename T>
-__global__ void k_products(Dims d, const T *__restrict__ vel, const T *__restrict__ vor, T *__restrict__ r,
-                           T *__restrict__ q, T *__restrict__ p)
-{
-    COLUMN_HEADER
-    const long long N = d.nfield;
-    for (int iz = threadIdx.x; iz <= d.nz; iz += 32) {
-        const long long i = o + iz;
-        const T u = vel[i], v = vel[N + i], w = vel[2 * N + i];
-        const T xi = vor[i], eta = vor[N + i], zeta = vor[2 * N + i];
-        r[i] = u * eta - v * xi;
-        q[i] = w * xi - u * zeta;
-        p[i] = v * zeta - w * eta;
-    }
-}
-template <typename T>
-void op_products(const Dims &d, cudaStream_t st, const T *vel, const T *vor, T *r, T *q, T *p)
-{
-    k_products<T><<<col_grid(d), COL_BLOCK, 0, st>>>(d, vel, vor, r, q, p);
-}
-
-// The products together with the z derivatives of q and p (central_diffz,
+// r = u eta - v xi, q = w xi - u zeta, p = v zeta - w eta (inversion.f90:
+// 327-352) together with the z derivatives of q and p (central_diffz,
 // inversion_utils.f90:653-673) in one pass over each column: the
 // neighbours iz -+ 1 come from the adjacent lanes, and across 32-level
 // chunks from the previous chunk (carried) or the next one, whose products
 // are formed before this chunk's derivatives.  One difference and one
 // product per derivative for all lanes alike: lane-dependent branches cost
-// the FP64 form a pass of its pipe each (256^3: 754 us with them, 361 now).  Same
-// arithmetic as k_products followed by k_diffz.
+// the FP64 form a pass of its pipe each (256^3: 754 us with them, 361 now).  The
+// arithmetic of k_diffz on the products.
 template <typename T>
 __global__ void k_products_dz(Dims d, T dzi, T hdzi, const T *__restrict__ vel, const T *__restrict__ vor,
                               T *__restrict__ r, T *__restrict__ q, T *__restrict__ p, T *__restrict__ gq,
@@ -1966,7 +1945,6 @@ void op_hyperbolic_tables(const Dims &d, cudaStream_t st, const double *k2l2, co
     template void op_v2v_uv<T>(const Dims &, cudaStream_t, const Deriv &, const double *, const T *,           \
                                const T *, const double *, const double *, T *, T *);                           \
     template void op_add_const<T>(const Dims &, cudaStream_t, T *, double);                                    \
-    template void op_products<T>(const Dims &, cudaStream_t, const T *, const T *, T *, T *, T *);             \
     template void op_svorts<T>(const Dims &, cudaStream_t, const Deriv &, const T *, const T *, const T *,     \
                                const T *, const T *, T *, T *, T *);                                           \
     template void op_strain_fields<T>(const Dims &, cudaStream_t, const Deriv &, const T *, T *);              \
