@@ -294,19 +294,19 @@ __global__ void __launch_bounds__(LinePlan<N, INV, W>::T, LinePlan<N, INV, W>::M
     const int zt = t.level(p);
     const bool valid = zt < P && t.has(p, tiling.nbatch);  // P is a multiple of 8: both lanes or neither
     const long long base = t.batch * batch_stride + t.z0;  // floats
-    const long long mine = base + t.off(p, batch_stride);
+    const int off = TAILS<N> ? (int)t.off(p, batch_stride) : 4 * p;  // 3 batch strides at most, N < 512
     const float s = rsqrtf((float)N);
     constexpr int H = N / 2;
     const long long gs = line_stride >> 2;  // float4 units
     if (!INV) {
-        const float4 *gin = reinterpret_cast<const float4 *>(in + mine);
+        const float4 *gin = reinterpret_cast<const float4 *>(in + base) + (off >> 2);
         pass<N, 8, 1, false, W, true, false>(smL, gin, nullptr, gs, valid, 1.0f, tw, zv - zt);
         later_passes<N, false, W, false>(smL, nullptr, gs, valid, 1.0f, tw);
         if (!valid) return;
         // split the two packed real transforms of each lane and store the
         // Hermitian rows k and N - k (T is a multiple of PAIRS: every
         // thread stays on its quad)
-        float4 *o = reinterpret_cast<float4 *>(out + mine);
+        float4 *o = reinterpret_cast<float4 *>(out + base) + (off >> 2);
         for (int k = threadIdx.x / PAIRS; k <= H; k += T / PAIRS) {
             const float4 ck = smL[k * PAIRS + p];
             const float4 cn = smL[((N - k) & (N - 1)) * PAIRS + p];
@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(LinePlan<N, INV, W>::T, LinePlan<N, INV, W>::M
     } else {
         herm_first_pass<N, W>(reinterpret_cast<float2 *>(smL), in + base, line_stride >> 1, t, batch_stride,
                               tiling.nbatch, P, zv);
-        float4 *gout = reinterpret_cast<float4 *>(out + mine);
+        float4 *gout = reinterpret_cast<float4 *>(out + base) + (off >> 2);
         later_passes<N, true, W, true>(smL, gout, gs, valid, s, tw);
     }
 }
@@ -383,7 +383,8 @@ __global__ void __launch_bounds__(LinePlan<N, false, W>::T, LinePlan<N, false, W
     const bool valid = zt < P && t.has(p, tiling.nbatch);  // P is a multiple of 8: all four or none
     // first and last quad of a run of levels: their outer neighbours are loaded
     const bool first = t.tail ? !(p & 1) : p == 0, last = t.tail ? (p & 1) : p == PAIRS - 1;
-    const long long base = t.batch * batch_stride + t.z0 + t.off(p, batch_stride);
+    const long long base = t.batch * batch_stride + t.z0;
+    const int off = TAILS<N> ? (int)t.off(p, batch_stride) : 4 * p;  // 3 batch strides at most, N < 512
     const long long Nf = ps.nfield;
     const float *u = ps.vel, *v = ps.vel + Nf, *w = ps.vel + 2 * Nf;
     const float *xi = ps.vor, *eta = ps.vor + Nf, *zeta = ps.vor + 2 * Nf;
@@ -425,7 +426,7 @@ __global__ void __launch_bounds__(LinePlan<N, false, W>::T, LinePlan<N, false, W
     // the product at (row, levels zt..zt+3); blocks 1, 2 write its z
     // derivative there to their derivative's output tile
     auto load = [&](int row) -> float4 {
-        const long long i = base + (long long)row * line_stride;
+        const long long i = base + (long long)row * line_stride + off;
         const float4 f = valid ? prod4(i) : make_float4(0.f, 0.f, 0.f, 0.f);
         if (o) {
             // neighbours zt - 1 and zt + 4: from the threads beside this one
@@ -454,7 +455,7 @@ __global__ void __launch_bounds__(LinePlan<N, false, W>::T, LinePlan<N, false, W
     // Hermitian rows k and N - k (as k_lines32)
     auto store = [&](float *dst) {
         if (!valid) return;
-        float4 *ob = reinterpret_cast<float4 *>(dst + base);
+        float4 *ob = reinterpret_cast<float4 *>(dst + base) + (off >> 2);
         for (int k = g; k <= H; k += T / PAIRS) {
             const float4 ck = smL[k * PAIRS + p];
             const float4 cn = smL[((N - k) & (N - 1)) * PAIRS + p];
@@ -499,7 +500,7 @@ __global__ void __launch_bounds__(LinePlan<N, false, W>::T, LinePlan<N, false, W
     // the derivative: each thread reads back the values it parked (its own
     // rows and levels), then the same transform in place
     __syncthreads();
-    const float4 *gin = reinterpret_cast<const float4 *>(dout + base);
+    const float4 *gin = reinterpret_cast<const float4 *>(dout + base) + (off >> 2);
     pass<N, 8, 1, false, W, true, false>(smL, gin, nullptr, gs, valid, 1.0f, tw, nval);
     later_passes<N, false, W, false>(smL, nullptr, gs, valid, 1.0f, tw);
     store(dout);
