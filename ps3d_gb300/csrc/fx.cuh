@@ -6,8 +6,11 @@
 // into 64-bit integers on one scale per line (its largest magnitude), the
 // FFT runs on the integer pipes, and the outputs go back to FP64.  Sums are
 // exact; a product with a twiddle keeps 63 bits, so the rounding of a whole
-// transform stays below that of an FP64 FFT (errors relative to the line's
-// norm against 80-bit sums, tests/test_fx_transforms.py).
+// transform stays below that of the FP64 Stockham transforms it stands for, at
+// every length they serve (mean over random lines of the error relative to the
+// line's norm, 0.1 to 0.85 of theirs: tests/test_fx_accuracy.py).  A unit is
+// common to a line, so single lines can be above: entries far below its largest
+// hold fewer bits than FP64.
 //
 // Everything here is plain integer arithmetic, compiled for host and device:
 // the host build of the same functions is what the CPU test runs.
@@ -208,11 +211,16 @@ FX_FN constexpr int up_shift(int r) { return r <= 5 ? 1 : 0; }
 // leaves one bit for the sum of two outputs that separates a forward pair
 // and for the doubled input of a small radix.  A modulus after the passes of product p
 // is bounded by p times the largest input and by the sum over the line's
-// inputs: l = ceil(log2(sum / largest)) is measured per line, so that a
-// line with a few large entries (a decaying spectrum) keeps more bits.
+// inputs: l, the least with sum < 2^(l + e + 1), is measured per line, so that
+// a line with a few large entries (a decaying spectrum) keeps more bits.  It
+// counts from 2^(e+1) as the unit does: counted from the largest magnitude
+// it allows for up to a bit that is not there, in the lines whose largest
+// value lies just above 2^e and whose unit is coarsest as it is.
 // Two real lines go as a + i b: moduli up to 2^(E+1/2), sums 2^(E+1+l); a
 // pair of Hermitian spectra one bit more of each; a column pair is folded
-// first (sums of four terms, then a quarter of them).
+// first: sums of four terms, then a quarter of them.  Every input enters two
+// terms of a folded sequence (the middle one a doubled term), so a sequence
+// sums to at most half of what the columns do: 2^(E+l).
 constexpr int MAXL = 13;
 struct Plan {
     signed char E[MAXL];  // bits for l = 0..MAXL-1
@@ -238,7 +246,7 @@ inline Plan make_plan(int n, int mode, int inputs, double scale2)
             rem /= r;
             lp += log2((double)r);
             if (passes) down += 2.0 - up_shift(r);
-            top = fmax(top, fmin(lp + m, l + sm) - down);
+            top = fmax(top, fmin(lp + m, mode == 2 ? l : l + sm) - down);
         }
         pl.E[l] = (signed char)(int)floor(61.5 - top + 1e-9);
     }
@@ -359,19 +367,21 @@ FX_FN float magf(unsigned m)
     return c.f;
 #endif
 }
-// l of a line from the FP32 sum of its magnitudes and its largest word (the
-// bound lcap where FP32 does not reach)
+// l of a line from the FP32 sum of its magnitudes (rounded, of truncated
+// words: raised by 1/1000) and its largest word; the bound lcap where FP32
+// does not reach
 FX_FN int spread(float sum, unsigned m, int lcap)
 {
     if (m < (933u << 20) || m > (1123u << 20)) return lcap;
-    const float r = sum * 1.001f / magf(m);
+    const float r = sum * 1.001f;
 #ifdef __CUDA_ARCH__
-    const int l = (__float_as_int(r) >> 23) - 126;
+    const int q = __float_as_int(r);
 #else
     union { float f; int i; } c;
     c.f = r;
-    const int l = (c.i >> 23) - 126;
+    const int q = c.i;
 #endif
+    const int l = (q >> 23) + 896 - (int)(m >> 20);  // floor(log2 r) - e
     return l < 0 ? 0 : l > lcap ? lcap : l;
 }
 // how a line's fixed-point outputs go back: v c 2^k
