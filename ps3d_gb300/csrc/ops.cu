@@ -1373,13 +1373,17 @@ void op_mean_fix(const Dims &d, cudaStream_t st, double *svor, const double *dst
 // Knuth two-sum in FP32 registers for the mixed form, so its error is that
 // of an FP64 sum without FP64 arithmetic per element), then an FP64 tree
 // across threads and a fixed-order FP64 compensated sum across blocks.
+// The larger of sum and term is told by the upper words on the integer pipe
+// (where those agree the exponents do, and either order gives the exact
+// error): four FP64 operations per term instead of six.
 struct KSum {
     double s, c;
     __device__ void add(double v)
     {
         const double t = s + v;
-        if (fabs(s) >= fabs(v)) c += (s - t) + v;
-        else c += (v - t) + s;
+        const bool swap = (__double2hiint(v) & 0x7fffffff) > (__double2hiint(s) & 0x7fffffff);
+        const double a = swap ? v : s, b = swap ? s : v;
+        c += (a - t) + b;
         s = t;
     }
     __device__ double value() const { return s + c; }
@@ -1512,10 +1516,9 @@ __global__ void k_red1(Dims d, const T *__restrict__ vel, const T *__restrict__ 
     block_reduce_store<RED1_N>(vals, kinds, part);
 }
 
-// The FP64 form of pass 1: the sums of a lane's elements of one column are
-// plain fma chains and enter the compensated accumulators once per column,
-// and the maxima compare bit patterns.  The FP64 pipe bounds it: 15
-// operations per element instead of about 50; 256^3: 2174 -> 658 us.
+// The FP64 form of pass 1: the maxima compare bit patterns and only the end
+// levels are halved; every term enters its compensated accumulator.  The FP64
+// pipe bounds it (33 operations per element instead of about 50).
 __device__ __forceinline__ long long order_key(double x)
 {
     const long long b = __double_as_longlong(x);
@@ -1540,31 +1543,31 @@ __global__ void k_red1<double>(Dims d, const double *__restrict__ vel, const dou
     for (long long col = (long long)blockIdx.x * COLS_PER_BLOCK + threadIdx.y; col < d.ncol;
          col += (long long)gridDim.x * COLS_PER_BLOCK) {
         const long long o = col * d.P;
-        double w2c = 0.0, u2c = 0.0, hc = 0.0, m0c = 0.0, m1c = 0.0, m2c = 0.0;
 #pragma unroll 2
         for (int iz = threadIdx.x; iz <= d.nz; iz += 32) {
             const long long i = o + iz;
-            const double wt = (iz == 0 || iz == d.nz) ? 0.5 : 1.0;
-            const double x = vor[i], y = vor[N + i], z = vor[2 * N + i];
+            double x = vor[i], y = vor[N + i], z = vor[2 * N + i];
             const double u = vel[i], v = vel[N + i], w = vel[2 * N + i];
-            const double w2 = x * x + y * y + z * z;
+            double w2 = x * x + y * y + z * z, u2 = u * u + v * v + w * w, h = u * x + v * y + w * z;
             raise(wmax2, w2);
-            w2c += wt * w2;
-            u2c += wt * (u * u + v * v + w * w);
-            hc += wt * (u * x + v * y + w * z);
-            m0c += wt * x;
-            m1c += wt * y;
-            m2c += wt * z;
             raise(vmx[0], u);
             raise(vmx[1], v);
             raise(vmx[2], w);
+            if (iz == 0 || iz == d.nz) {
+                w2 *= 0.5;
+                u2 *= 0.5;
+                h *= 0.5;
+                x *= 0.5;
+                y *= 0.5;
+                z *= 0.5;
+            }
+            s_w2.add(w2);
+            s_u2.add(u2);
+            s_h.add(h);
+            s_m0.add(x);
+            s_m1.add(y);
+            s_m2.add(z);
         }
-        s_w2.add(w2c);
-        s_u2.add(u2c);
-        s_h.add(hc);
-        s_m0.add(m0c);
-        s_m1.add(m1c);
-        s_m2.add(m2c);
     }
     double vals[RED1_N] = {key_value(wmax2), s_w2.value(), s_u2.value(), s_h.value(), s_m0.value(), s_m1.value(),
                            s_m2.value(), key_value(vmx[0]), key_value(vmx[1]), key_value(vmx[2]), 0.0, 0.0};
@@ -1760,7 +1763,6 @@ __global__ void k_red2_screen(Dims d, const double *__restrict__ vor, const doub
     for (long long col = (long long)blockIdx.x * COLS_PER_BLOCK + threadIdx.y; col < d.ncol;
          col += (long long)gridDim.x * COLS_PER_BLOCK) {
         const long long o = col * d.P;
-        double s1 = 0.0, s2 = 0.0;  // of twice the mid-level magnitudes
         for (int c0 = 0; c0 <= d.nz; c0 += 32) {
             const int iz = c0 + threadIdx.x;
             float e = 0.0f;
@@ -1770,9 +1772,9 @@ __global__ void k_red2_screen(Dims d, const double *__restrict__ vor, const doub
                     const double v1 = vor[i - 1] + vor[i], v2 = vor[N + i - 1] + vor[N + i],
                                  v3 = vor[2 * N + i - 1] + vor[2 * N + i];
                     const double s = fabs(v1) + fabs(v2) + fabs(v3);
-                    if (s > vr2) {
-                        s1 += s;
-                        s2 += v1 * v1 + v2 * v2 + v3 * v3;
+                    if (s > vr2) {  // sums of twice the mid-level magnitudes
+                        l1.add(s);
+                        l2.add(v1 * v1 + v2 * v2 + v3 * v3);
                     }
                 }
                 e = strain_estimate(strain_point(vor, g5, N, i));
@@ -1791,10 +1793,8 @@ __global__ void k_red2_screen(Dims d, const double *__restrict__ vor, const doub
             const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(e));
             if (threadIdx.x == 0) est[col * ep + (c0 >> 5)] = __uint_as_float(m);
         }
-        l1.add(0.5 * s1);
-        l2.add(0.25 * s2);
     }
-    double vals[RED2_N] = {l1.value(), l2.value(), (double)gg, (double)us, (double)ls};
+    double vals[RED2_N] = {0.5 * l1.value(), 0.25 * l2.value(), (double)gg, (double)us, (double)ls};
     const int kinds[RED2_N] = {0, 0, 1, 1, 1};
     block_reduce_store<RED2_N>(vals, kinds, part);
 }
