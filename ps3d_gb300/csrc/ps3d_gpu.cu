@@ -10,8 +10,6 @@
 // transient fields with FP64 prognostic vorticity, RK accumulators,
 // low-mode inversion and reductions).
 #include <cuda_runtime.h>
-#include <sys/mman.h>
-#include <unistd.h>
 
 #include <atomic>
 #include <cmath>
@@ -19,10 +17,10 @@
 #include <cstdlib>
 #include <cstring>
 #include <string>
-#include <thread>
 #include <vector>
 
 #include "../../include/ps3d_gpu.h"
+#include "host_pages.h"
 #include "kernels.h"
 
 using namespace ps3d;
@@ -254,46 +252,6 @@ int upload(ps3d_gpu_ctx *c, const double *h, int ncomp, void *dst, bool dst_is_f
         }
     }
     return check(c, "upload");
-}
-
-// Pages of a fresh host array (numpy's zeros, calloc) exist only after their
-// first write, and the driver's copy into them faults page by page: 43 ms for
-// the 51 MB of a 128^3 state, against 1 ms into pages that exist.  The pages
-// are made first, by a few threads (MADV_POPULATE_WRITE keeps their
-// contents; where the kernel lacks it, or for memory it does not take, the
-// copy works as before).  From 8 MB on: smaller arrays come from heap pages
-// that were in use before, and copy in well under a millisecond.
-void populate(void *p, size_t bytes)
-{
-#ifdef MADV_POPULATE_WRITE
-    constexpr size_t MIN = (size_t)8 << 20, PART = (size_t)4 << 20;
-    if (bytes < MIN) return;
-    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
-    char *a = (char *)(((uintptr_t)p + page - 1) / page * page);
-    char *e = (char *)(((uintptr_t)p + bytes) / page * page);
-    // an array that was written before has its pages: 16 of them tell
-    bool fresh = false;
-    for (int i = 0; i < 16 && !fresh; ++i) {
-        unsigned char in = 1;
-        char *q = a + (size_t)(e - a - 1) / 16 * i / page * page;
-        fresh = mincore(q, page, &in) != 0 || !(in & 1);
-    }
-    if (!fresh) return;
-    std::atomic<size_t> next{0};
-    const auto work = [&] {
-        for (size_t o; (o = next.fetch_add(PART)) < (size_t)(e - a);) {
-            const size_t n = (size_t)(e - a) - o < PART ? (size_t)(e - a) - o : PART;
-            if (madvise(a + o, n, MADV_POPULATE_WRITE)) return;
-        }
-    };
-    std::vector<std::thread> t;
-    try {
-        for (int i = 0; i < 7; ++i) t.emplace_back(work);
-    } catch (...) {  // no more threads: the ones that run do the work
-    }
-    work();
-    for (std::thread &x : t) x.join();
-#endif
 }
 
 int download(ps3d_gpu_ctx *c, const void *src, bool src_is_fp64, int ncomp, double *h)
