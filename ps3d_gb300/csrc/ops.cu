@@ -1084,6 +1084,8 @@ __device__ __forceinline__ void chunk_pos(int e, int n1, float inv_n1, int &col,
     iz = e - col * n1;
 }
 
+// changed null: no comparison, and the destination (which a first upload finds
+// unset) is not read
 __global__ void __launch_bounds__(FLAT_T) k_unpack_flat(Dims d, const double2 *__restrict__ src,
                                                         double *__restrict__ dst, long long ncols, float inv_n1,
                                                         int *__restrict__ changed)
@@ -1093,6 +1095,7 @@ __global__ void __launch_bounds__(FLAT_T) k_unpack_flat(Dims d, const double2 *_
     const int ne = (int)min((long long)FLAT_COLS, ncols - c0) * n1;  // elements of this chunk
     const double2 *s = src + ((c0 * n1) >> 1);                         // c0 even: whole pairs
     double *t = dst + c0 * d.P;
+    const bool check = changed != nullptr;
     bool diff = false;
     for (int q0 = threadIdx.x; 2 * q0 < ne; q0 += FLAT_T * FLAT_U) {
         double2 v[FLAT_U];
@@ -1109,7 +1112,7 @@ __global__ void __launch_bounds__(FLAT_T) k_unpack_flat(Dims d, const double2 *_
                 int col, iz;
                 chunk_pos(e, n1, inv_n1, col, iz);
                 double *p0 = t + (long long)col * d.P + iz;
-                diff |= __double_as_longlong(v[u].x) != __double_as_longlong(*p0);
+                if (check) diff |= __double_as_longlong(v[u].x) != __double_as_longlong(*p0);
                 *p0 = v[u].x;
                 if (e + 1 < ne) {
                     if (++iz == n1) {
@@ -1117,13 +1120,13 @@ __global__ void __launch_bounds__(FLAT_T) k_unpack_flat(Dims d, const double2 *_
                         ++col;
                     }
                     double *p1 = t + (long long)col * d.P + iz;
-                    diff |= __double_as_longlong(v[u].y) != __double_as_longlong(*p1);
+                    if (check) diff |= __double_as_longlong(v[u].y) != __double_as_longlong(*p1);
                     *p1 = v[u].y;
                 }
             }
         }
     }
-    if (__any_sync(0xffffffffu, diff) && (threadIdx.x & 31) == 0) atomicOr(changed, 1);
+    if (check && __syncthreads_or(diff) && threadIdx.x == 0) atomicOr(changed, 1);
 }
 
 __global__ void __launch_bounds__(FLAT_T) k_pack_flat(Dims d, const double *__restrict__ src,
@@ -1224,7 +1227,7 @@ __global__ void k_unpack_cols(Dims d, const double *__restrict__ src, double *__
     bool diff = false;
     for (int iz = threadIdx.x; iz < n1; iz += 32) {
         const double v = s[iz];
-        diff |= __double_as_longlong(v) != __double_as_longlong(t[iz]);
+        if (changed) diff |= __double_as_longlong(v) != __double_as_longlong(t[iz]);
         t[iz] = v;
     }
     if (__any_sync(0xffffffffu, diff) && threadIdx.x == 0) atomicOr(changed, 1);

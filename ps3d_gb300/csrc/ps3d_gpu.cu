@@ -244,7 +244,7 @@ int upload(ps3d_gpu_ctx *c, const double *h, int ncomp, void *dst, bool dst_is_f
     for (int k = 0; k < ncomp; ++k) {
         if (cudaMemcpyAsync(lin, h + k * n, n * sizeof(double), cudaMemcpyHostToDevice, c->st) != cudaSuccess)
             return check(c, "upload");
-        op_unpack_cols(d, c->st, lin, dst_is_fp64 ? tf<double>(dst) + (size_t)k * d.nfield : c->stage64, 1, c->flag);
+        op_unpack_cols(d, c->st, lin, dst_is_fp64 ? tf<double>(dst) + (size_t)k * d.nfield : c->stage64, 1, nullptr);
         c->launches += 1;
         if (!dst_is_fp64) {
             op_convert<float, double>(d, c->st, c->stage64, tf<float>(dst) + (size_t)k * d.nfield, d.nfield);
@@ -2552,8 +2552,9 @@ int ps3d_gpu_advance_host(ps3d_gpu_ctx *c, double *svor, double *t, ps3d_gpu_dia
         }
     }
     if (!mapped) cudaMemcpyAsync(stage, svor, bytes, cudaMemcpyHostToDevice, c->st);
-    cudaMemsetAsync(c->flag, 0, sizeof(int), c->st);
-    op_unpack_cols(d, c->st, stage, c->svor, 3, c->flag);
+    // only the mixed form asks whether the state changed
+    if (!c->fp64) cudaMemsetAsync(c->flag, 0, sizeof(int), c->st);
+    op_unpack_cols(d, c->st, stage, c->svor, 3, c->fp64 ? nullptr : c->flag);
     c->launches += 1;
     if (!c->fp64) {
         // a state bitwise equal to the device's (the previous step's result)
