@@ -145,14 +145,15 @@ struct Tile {
     __device__ int level(int q) const { return z0 + (tail ? 4 * (q & 1) : 4 * q); }
     __device__ bool has(int q, long long nbatch) const { return !tail || batch + (q >> 1) < nbatch; }
 };
-// lines of 512 and more: tiles of their batch only, batches in the grid's y
-// (the general numbering cost their kernels registers: host step at 512^3
-// 72.3 -> 72.8 ms)
+// lines of 512 and more: tiles of their batch only, batches in the grid's y,
+// lanes and stores addressed from the tile's first level (the general
+// numbering cost their kernels registers: host step at 512^3 72.3 -> 72.8 ms;
+// with the general addressing alone a forward pass took 0.199 ms, 0.196 so)
 template <int N> constexpr bool TAILS = N < 512;
 struct Tiling {
     int full;          // 32-level tiles per batch
     long long nbatch;
-        __host__ __device__ static bool short_tail(int zv)
+    __host__ __device__ static bool short_tail(int zv)
     {
         return zv % 32 >= 1 && zv % 32 <= 8 && zv > 32 && zv <= 8 * 32 + 8;
     }
@@ -194,9 +195,10 @@ __device__ __forceinline__ void herm_first_pass(float2 *sm2, const float *__rest
         const int it = threadIdx.x + T * q;
         if (!(ITEMS % T == 0 || it < ITEMS)) continue;
         const int lane = it & (LANES - 1), s = it / LANES;
-        const int z = t.level(lane >> 1) + 2 * (lane & 1);
-        const bool valid = z < P && t.has(lane >> 1, nbatch);
-        const float2 *g = reinterpret_cast<const float2 *>(in + t.off(lane >> 1, bs)) + (lane & 1);
+        const int z = TAILS<N> ? t.level(lane >> 1) + 2 * (lane & 1) : t.z0 + 2 * lane;
+        const bool valid = z < P && (!TAILS<N> || t.has(lane >> 1, nbatch));
+        const float2 *g = TAILS<N> ? reinterpret_cast<const float2 *>(in + t.off(lane >> 1, bs)) + (lane & 1)
+                                   : reinterpret_cast<const float2 *>(in) + lane;
         const int j1 = s == 0 ? 0 : s, j2 = s == 0 ? NB / 2 : NB - s;
         float2 h1[8], h2[8];
 #pragma unroll
@@ -291,37 +293,54 @@ __global__ void __launch_bounds__(LinePlan<N, INV, W>::T, LinePlan<N, INV, W>::M
     constexpr int T = LinePlan<N, INV, W>::T;
     const int p = threadIdx.x & (PAIRS - 1);
     const Tile t = TAILS<N> ? tiling.tile(blockIdx.x) : Tile{(int)blockIdx.x * 2 * LANES, blockIdx.y, false};
-    const int zt = t.level(p);
-    const bool valid = zt < P && t.has(p, tiling.nbatch);  // P is a multiple of 8: both lanes or neither
+    const int zt = TAILS<N> ? t.level(p) : t.z0 + 4 * p;
+    const bool valid = zt < P && (!TAILS<N> || t.has(p, tiling.nbatch));  // P is a multiple of 8: both lanes or neither
     const long long base = t.batch * batch_stride + t.z0;  // floats
-    const int off = TAILS<N> ? (int)t.off(p, batch_stride) : 4 * p;  // 3 batch strides at most, N < 512
+    // the thread's quad from there (3 batch strides away at most, N < 512)
+    const int quad = TAILS<N> ? (int)t.off(p, batch_stride) >> 2 : p;
     const float s = rsqrtf((float)N);
     constexpr int H = N / 2;
     const long long gs = line_stride >> 2;  // float4 units
     if (!INV) {
-        const float4 *gin = reinterpret_cast<const float4 *>(in + base) + (off >> 2);
+        const float4 *gin = reinterpret_cast<const float4 *>(in + base) + quad;
         pass<N, 8, 1, false, W, true, false>(smL, gin, nullptr, gs, valid, 1.0f, tw, zv - zt);
         later_passes<N, false, W, false>(smL, nullptr, gs, valid, 1.0f, tw);
-        if (!valid) return;
         // split the two packed real transforms of each lane and store the
-        // Hermitian rows k and N - k (T is a multiple of PAIRS: every
-        // thread stays on its quad)
-        float4 *o = reinterpret_cast<float4 *>(out + base) + (off >> 2);
-        for (int k = threadIdx.x / PAIRS; k <= H; k += T / PAIRS) {
-            const float4 ck = smL[k * PAIRS + p];
-            const float4 cn = smL[((N - k) & (N - 1)) * PAIRS + p];
-            // lane 0 in (x, y), lane 1 in (z, w); A = real line z, B = z + 1
-            const float4 re = make_float4(0.5f * (ck.x + cn.x) * s, 0.5f * (ck.y + cn.y) * s,
-                                          0.5f * (ck.z + cn.z) * s, 0.5f * (ck.w + cn.w) * s);
-            o[k * gs] = re;
-            if (k > 0 && k < H)
-                o[(N - k) * gs] = make_float4(0.5f * (ck.y - cn.y) * s, -0.5f * (ck.x - cn.x) * s,
-                                              0.5f * (ck.w - cn.w) * s, -0.5f * (ck.z - cn.z) * s);
+        // Hermitian rows k and N - k; lane 0 in (x, y), lane 1 in (z, w);
+        // A = real line z, B = z + 1
+        if constexpr (TAILS<N>) {
+            // T is a multiple of PAIRS: every thread stays on its quad
+            if (!valid) return;
+            float4 *o = reinterpret_cast<float4 *>(out + base) + quad;
+            for (int k = threadIdx.x / PAIRS; k <= H; k += T / PAIRS) {
+                const float4 ck = smL[k * PAIRS + p];
+                const float4 cn = smL[((N - k) & (N - 1)) * PAIRS + p];
+                const float4 re = make_float4(0.5f * (ck.x + cn.x) * s, 0.5f * (ck.y + cn.y) * s,
+                                              0.5f * (ck.z + cn.z) * s, 0.5f * (ck.w + cn.w) * s);
+                o[k * gs] = re;
+                if (k > 0 && k < H)
+                    o[(N - k) * gs] = make_float4(0.5f * (ck.y - cn.y) * s, -0.5f * (ck.x - cn.x) * s,
+                                                  0.5f * (ck.w - cn.w) * s, -0.5f * (ck.z - cn.z) * s);
+            }
+        } else {
+            float4 *o = reinterpret_cast<float4 *>(out + base);
+            for (int e = threadIdx.x; e < (H + 1) * PAIRS; e += T) {
+                const int k = e / PAIRS, q = e & (PAIRS - 1);
+                if (t.z0 + 4 * q >= P) continue;
+                const float4 ck = smL[k * PAIRS + q];
+                const float4 cn = smL[((N - k) & (N - 1)) * PAIRS + q];
+                const float4 re = make_float4(0.5f * (ck.x + cn.x) * s, 0.5f * (ck.y + cn.y) * s,
+                                              0.5f * (ck.z + cn.z) * s, 0.5f * (ck.w + cn.w) * s);
+                o[k * gs + q] = re;
+                if (k > 0 && k < H)
+                    o[(N - k) * gs + q] = make_float4(0.5f * (ck.y - cn.y) * s, -0.5f * (ck.x - cn.x) * s,
+                                                      0.5f * (ck.w - cn.w) * s, -0.5f * (ck.z - cn.z) * s);
+            }
         }
     } else {
         herm_first_pass<N, W>(reinterpret_cast<float2 *>(smL), in + base, line_stride >> 1, t, batch_stride,
                               tiling.nbatch, P, zv);
-        float4 *gout = reinterpret_cast<float4 *>(out + base) + (off >> 2);
+        float4 *gout = reinterpret_cast<float4 *>(out + base) + quad;
         later_passes<N, true, W, true>(smL, gout, gs, valid, s, tw);
     }
 }
