@@ -472,37 +472,49 @@ void fx_columns(const Dims &d, cudaStream_t st, int mode, const double *in, doub
         else go(k_fx_columns<COL_COMBINE, NIT, LB>);
     });
 }
+// bytes of nf fields, for the probe
+static double field_bytes(const Dims &d, int nf)
+{
+    return (double)nf * (double)d.ncol * (double)(d.nz + 1) * sizeof(double);
+}
+
 void fx_comdec(const Dims &d, cudaStream_t st, const double *c, double *cs, double *es, double dzi,
-               const double *phim, const double *phip, const void *tw)
+               const double *phim, const double *phip, const void *tw, Probe *pr)
 {
     const fx::Plan pl = fx::col_plan(d.nz);
+    if (pr) pr->begin(PROBE_COLUMNS, st);
     col_shape(d.nz, d.ncol, [&](auto nit, auto lb) {
         constexpr int NIT = decltype(nit)::value, LB = decltype(lb)::value;
         k_fx_comdec<NIT, LB><<<col_grid(d, LB, 1), 256, (size_t)d.nz * 48 << LB, st>>>(
             c, cs, es, d.nz, d.P, d.ncol, dzi, phim, phip, pl, reinterpret_cast<const Tw *>(tw));
     });
+    if (pr) pr->end(PROBE_COLUMNS, st, field_bytes(d, 3));
 }
 void fx_w(const Dims &d, cudaStream_t st, const double *A, const double *B, double *w, double *es, const Deriv &D,
           const double *thetam, const double *thetap, const double *dthetam, const double *dthetap,
-          const double *green, const double *rkz, const void *tw)
+          const double *green, const double *rkz, const void *tw, Probe *pr)
 {
     const fx::Plan pl = fx::col_plan(d.nz);
+    if (pr) pr->begin(PROBE_COLUMNS, st);
     const WTables tb{thetam, thetap, dthetam, dthetap, green, rkz};
     col_shape(d.nz, d.ncol, [&](auto nit, auto lb) {
         constexpr int NIT = decltype(nit)::value, LB = decltype(lb)::value;
         k_fx_w<NIT, LB><<<col_grid(d, LB, 1), 256, (size_t)d.nz * 48 << LB, st>>>(
             A, B, w, es, d.nx, d.ny, d.nz, d.P, d.ncol, D, tb, pl, reinterpret_cast<const Tw *>(tw));
     });
+    if (pr) pr->end(PROBE_COLUMNS, st, field_bytes(d, 4));
 }
 void fx_src(const Dims &d, cudaStream_t st, const double *f, double *out, const Deriv &D, const double *phim,
-            const double *phip, const void *tw)
+            const double *phip, const void *tw, Probe *pr)
 {
     const fx::Plan pl = fx::col_plan(d.nz);
+    if (pr) pr->begin(PROBE_COLUMNS, st);
     col_shape(d.nz, d.ncol, [&](auto nit, auto lb) {
         constexpr int NIT = decltype(nit)::value, LB = decltype(lb)::value;
         k_fx_src<NIT, LB><<<col_grid(d, LB, 3), 256, (size_t)d.nz * 48 << LB, st>>>(
             f, out, d.nx, d.ny, d.nz, d.P, d.ncol, d.nfield, D, phim, phip, pl, reinterpret_cast<const Tw *>(tw));
     });
+    if (pr) pr->end(PROBE_COLUMNS, st, field_bytes(d, 8));
 }
 
 void fx_columns_init()

@@ -103,12 +103,12 @@ void fx_columns_init();
 // state components; the tendency components of five consecutive transformed
 // products, decomposed
 void fx_comdec(const Dims &d, cudaStream_t st, const double *c, double *cs, double *es, double dzi,
-               const double *phim, const double *phip, const void *tw);
+               const double *phim, const double *phip, const void *tw, Probe *pr);
 void fx_w(const Dims &d, cudaStream_t st, const double *A, const double *B, double *w, double *es,
           const struct Deriv &D, const double *thetam, const double *thetap, const double *dthetam,
-          const double *dthetap, const double *green, const double *rkz, const void *tw);
+          const double *dthetap, const double *green, const double *rkz, const void *tw, Probe *pr);
 void fx_src(const Dims &d, cudaStream_t st, const double *f, double *out, const struct Deriv &D, const double *phim,
-            const double *phip, const void *tw);
+            const double *phip, const void *tw, Probe *pr);
 // FP32 bandwidth-tuned line FFTs (lines32.cu), n = 64..1024
 bool lines32_supported(int n);
 void lines32_init();

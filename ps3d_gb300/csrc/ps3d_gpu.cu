@@ -351,18 +351,19 @@ double *scratch64(ps3d_gpu_ctx *c, int i)
 }
 
 // es = decompose(diffz(cs)), cs = combine(C) (inversion.f90:41-47).  step:
-// inside a step (vor2vel of the FP64 form, the re-projection of mixed cn2)
-void combine_diffz64(ps3d_gpu_ctx *c, const double *Cc, double *cs, double *es, bool step)
+// inside a step (vor2vel of the FP64 form, the re-projection of mixed cn2);
+// pr: the probe that counts the column transforms, where they are counted
+void combine_diffz64(ps3d_gpu_ctx *c, const double *Cc, double *cs, double *es, bool step, Probe *pr)
 {
     const Dims &d = c->d;
     if (step && fx_serves(d.nz)) {
-        fx_comdec(d, c->st, Cc, cs, es, c->dzi, c->phim64, c->phip64, c->twz2_fx);
+        fx_comdec(d, c->st, Cc, cs, es, c->dzi, c->phim64, c->phip64, c->twz2_fx, pr);
         c->launches += 1;
         return;
     }
-    columns<double>(d, c->st, COL_COMBINE, Cc, cs, c->phim64, c->phip64, c->twz2_64, nullptr);
+    columns<double>(d, c->st, COL_COMBINE, Cc, cs, c->phim64, c->phip64, c->twz2_64, pr);
     op_diffz<double>(d, c->st, c->dzi, cs, es);
-    columns<double>(d, c->st, COL_DECOMP, es, es, c->phim64, c->phip64, c->twz2_64, nullptr);
+    columns<double>(d, c->st, COL_DECOMP, es, es, c->phim64, c->phip64, c->twz2_64, pr);
     c->launches += 3;
 }
 
@@ -376,7 +377,7 @@ void project64(ps3d_gpu_ctx *c, bool step)
     double *A = c->svor, *B = c->svor + N, *Cc = c->svor + 2 * N;
     double *cs = scratch64(c, 0), *es = scratch64(c, 1), *ds = scratch64(c, 2);
     op_v2v_ds<double, double>(d, c->st, c->D(), A, B, ds);
-    combine_diffz64(c, Cc, cs, es, step);
+    combine_diffz64(c, Cc, cs, es, step, nullptr);
     op_v2v_project<double, double>(d, c->st, c->D(), c->k2l2i, es, ds, A, B);
     c->launches += 2;
 }
@@ -417,7 +418,7 @@ int vor2vel_fp64(ps3d_gpu_ctx *c)
     const Deriv D = c->D();
 
     // solenoidal projection (inversion.f90:34-76)
-    combine_diffz64(c, Cc, cs, es, true);
+    combine_diffz64(c, Cc, cs, es, true, &c->probe);
     op_project64(d, c->st, D, c->k2l2i, es, A, B);
     c->launches += 1;
 
@@ -433,7 +434,7 @@ int vor2vel_fp64(ps3d_gpu_ctx *c)
     // vertical velocity (:86-139)
     if (fx_serves(d.nz)) {
         fx_w(d, c->st, A, B, svel + 2 * N, es, D, tf<T>(c->thetam), tf<T>(c->thetap), tf<T>(c->dthetam),
-             tf<T>(c->dthetap), tf<T>(c->green), c->rkz, c->twz2);
+             tf<T>(c->dthetap), tf<T>(c->green), c->rkz, c->twz2, &c->probe);
         c->launches += 1;
     } else {
         op_v2v_wsrc<T, double>(d, c->st, D, A, B, ds);
@@ -768,7 +769,7 @@ template <typename T> int source(ps3d_gpu_ctx *c)
     xyf<T>(c, r, r, 5);
     if constexpr (sizeof(T) == sizeof(double)) {
         if (fx_serves(d.nz)) {
-            fx_src(d, c->st, r, svorts, c->D(), tf<T>(c->phim), tf<T>(c->phip), c->twz2);
+            fx_src(d, c->st, r, svorts, c->D(), tf<T>(c->phim), tf<T>(c->phip), c->twz2, &c->probe);
             c->launches += 1;
         } else {
             op_svorts<T>(d, c->st, c->D(), r, q, p, gq, gp, svorts, svorts + N, svorts + 2 * N);
