@@ -671,9 +671,9 @@ __global__ void k_adam(float *__restrict__ w, const float *__restrict__ g, float
 // ===================================================== tcgen05 inference path
 // The forward pass on the 5th-generation tensor cores.  Activations live in a
 // padded, channel-chunk-planar layout: padded row r = GUARD + (iz+1) +
-// ZP*((iy+1) + YP*(ix+1)) (ZP = nz+3 rounded up to 8, YP = ny+2), chunk plane kc (8 channels,
+// ZP*((iy+1) + YP*(ix+1)) (ZP = nz+3, YP = ny+2), chunk plane kc (8 channels,
 // 16 bytes) at byte (kc*RTOT + r)*16.  Ghost rows at iz = -1, nz+1 stay zero
-// (the z zero padding, and what rounds ZP up); ghost rows at iy = -1, ny and ix = -1, nx hold the
+// (the z zero padding); ghost rows at iy = -1, ny and ix = -1, nx hold the
 // periodic copies, written by the producer of each activation; GUARD rows
 // before and after keep every load of a tile in bounds.  Every tap is then a
 // uniform shift of the row index, so one tile of 128 rows needs, per x shift
@@ -904,11 +904,14 @@ __device__ __forceinline__ void mbar_arrive(uint32_t a)
 // three dz taps of a neighbour column (dx, dy) are one product of N = 3 COUT:
 // D_dz(r) = sum over (dx, dy) of W_dz X(r), and the epilogue adds
 // D_-1(r - 1) + D_0(r) + D_+1(r + 1).  An operand row block is then read from
-// shared memory 9 times instead of 27, always from a multiple of 8 rows (ZP
-// is one): with 27 products of N = COUT that began at any row, shared-memory
-// reads of the rows bounded the layer (64^3: 32 -> 32 channels 60 us,
-// 16 -> 32 37, 32 -> 8 51; as one product, with two buffers and eight epilogue
-// warps, 44, 36 and 38; with three or four buffers and sixteen, 41, 32 and 32).
+// shared memory 9 times instead of 27: with 27 products of N = COUT,
+// shared-memory reads of the rows bounded the layer (64^3: 32 -> 32 channels
+// 60 us, 16 -> 32 37, 32 -> 8 51; as one product, with two buffers and eight
+// epilogue warps, 44, 36 and 38; with three or four buffers and sixteen, 41, 32
+// and 32).  ZP is not rounded to the 8 rows of a core matrix: the rows that
+// would add cost more than the alignment of the shifts gives (four forward
+// passes, rounded and not: 64^3 0.745 and 0.720 ms, 128x128x8 0.702 and 0.507,
+// 256x256x16 2.89 and 2.41).
 //
 // Warp 16 (one elected lane) is the producer and issuer: TMA copies of tile
 // k-1+nbuf into the shared buffer freed by the products of tile k-1 (two
@@ -1550,9 +1553,7 @@ int ps3d_closure_create(int nx, int ny, int nz, int max_samples, int device, uns
     cudaFuncSetAttribute(k_wgrad<32, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * WG<32, 16>::BUF);
     // tcgen05 path: padded geometry; available when a tile's shared memory
     // (weights + 3 x 4 chunk planes of 128 + 2 ZP rows) fits a block
-    // z pitch of a padded column: a multiple of 8 where a tile then still fits
-    cl->ZP = (nz + 3 + 7) / 8 * 8;
-    if (tc_smem<32, 32>(cl->ZP) + TC_STATIC > (size_t)prop.sharedMemPerBlockOptin) cl->ZP = nz + 3;
+    cl->ZP = nz + 3;
     cl->YP = ny + 2;
     cl->QN = (long long)(nx + 2) * cl->YP * cl->ZP;
     cl->GUARD = (long long)cl->YP * cl->ZP + cl->ZP + 256;
