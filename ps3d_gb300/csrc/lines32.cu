@@ -132,7 +132,8 @@ __device__ __forceinline__ void pass(float4 *sm, const float4 *__restrict__ gin,
 // 32 floats is 4 x 8 levels, 32 bytes of each.  Blocks are numbered z-tile
 // fastest, the tail blocks last.  5 tiles per batch become 4.25 at 128
 // levels: captured 128^3 step 1.271 -> 1.256 ms, batch of twelve runs
-// 88.5 -> 85.9 ms; 256^3 step 6.84 -> 6.77.  Above 264 levels the tail stays a
+// 88.5 -> 85.9 ms; 256^3 step 6.576 ms without, 6.512 with (6.504 before the
+// general numbering), 256x256x192 10.08 and 9.99.  Above 264 levels the tail stays a
 // tile of its batch: at 512^3 the gain of 17 -> 16.25 tiles is lost again by
 // reading those 32-byte pieces apart from their rows (host step 72.4 -> 73.2).
 struct Tile {
