@@ -164,7 +164,7 @@ static void launch_fx_lines(cudaStream_t st, const double *in, double *out, int 
     const fx::Plan pl = fx::line_plan(n, inverse);
     const int nt = (((n / R1) << LB) + 31) / 32 * 32;
     const dim3 grid((zv + (2 << LB) - 1) / (2 << LB), (unsigned)nbatch, (unsigned)nf);
-    const size_t sm = (size_t)n * 16 * BUFS << LB;  // at most 37 KB
+    const size_t sm = (size_t)n * 16 * BUFS << LB;  // at most 32 KB
     if (inverse)
         k_fx_lines<R1, T, true, LB, BUFS><<<grid, nt, sm, st>>>(in, out, n, P, zv, line_stride, batch_stride, fs_in,
                                                                 fs_out, pl, tw);
@@ -197,7 +197,7 @@ void fx_lines(cudaStream_t st, const double *in, double *out, int n, int P, int 
     else if (r == 8 && two) go(launch_fx_lines<8, 128, 2, 2>);
     else if (r == 8 && t <= 128) go(launch_fx_lines<8, 128, 2>);
     else if (r == 8) go(launch_fx_lines<8, 256, 2>);
-    else if (r == 4 && wide) two ? go(launch_fx_lines<4, 256, 3, 2>) : go(launch_fx_lines<4, 256, 3, 1>);
+    else if (r == 4 && wide) go(launch_fx_lines<4, 256, 3, 2>);  // at most 124 points
     else if (r == 4 && two) go(launch_fx_lines<4, 128, 2, 2>);
     else if (r == 4 && t <= 256) go(launch_fx_lines<4, 256, 2>);
     else if (r == 4) go(launch_fx_lines<4, 512, 2>);

@@ -322,24 +322,6 @@ void col64(ps3d_gpu_ctx *c, int mode, const double *in, double *out, int nf)
                     &c->probe, nf);
     c->launches += c->d.fx64 && fx_serves(c->d.nz) ? 1 : nf;
 }
-// a T view of an FP64 state component (copy for the mixed form)
-template <typename T> const T *state_as_T(ps3d_gpu_ctx *c, const double *s, T *scratch)
-{
-    if (sizeof(T) == sizeof(double)) return reinterpret_cast<const T *>(s);
-    op_convert<float, double>(c->d, c->st, s, reinterpret_cast<float *>(scratch), c->d.nfield);
-    c->launches += 1;
-    return scratch;
-}
-template <typename T> void state_from_T(ps3d_gpu_ctx *c, const T *src, double *s)
-{
-    if (sizeof(T) == sizeof(double)) {
-        if ((const void *)src != (const void *)s)
-            cudaMemcpyAsync(s, src, c->d.nfield * sizeof(double), cudaMemcpyDeviceToDevice, c->st);
-        return;
-    }
-    op_convert<double, float>(c->d, c->st, reinterpret_cast<const float *>(src), s, c->d.nfield);
-    c->launches += 1;
-}
 
 // FP64 scratch fields for the FP64 projection: the FP64 form uses its
 // transient temporaries, the mixed form the RK accumulator svorf (free
