@@ -141,31 +141,6 @@ def peaks():
         return 6800.0, "fallback"
 
 
-def fp64_peak_tflops(dev):
-    """FP64 peak of this GPU as measured by a cuBLAS DGEMM through torch
-    (plumbing: 2 n^3 flops per 4096^3 product, best of 5)."""
-    try:
-        import torch
-        n = 4096
-        a = torch.randn(n, n, dtype=torch.float64, device=f"cuda:{dev}")
-        b = torch.randn(n, n, dtype=torch.float64, device=f"cuda:{dev}")
-        torch.matmul(a, b)
-        best = None
-        for _ in range(5):
-            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-            e0.record()
-            torch.matmul(a, b)
-            e1.record()
-            torch.cuda.synchronize()
-            ms = e0.elapsed_time(e1)
-            best = ms if best is None else min(best, ms)
-        del a, b
-        torch.cuda.empty_cache()
-        return 2.0 * n ** 3 / (best * 1e-3) / 1e12
-    except Exception:
-        return None
-
-
 def cufft_comparator(n, dev):
     """cuFFT (torch.fft.rfft2 / irfft2 over x and y of an (n, n, P) FP32 field,
     z contiguous as here) timed as a comparator for one forward and one
@@ -466,18 +441,16 @@ def run_gpu(args, rank, world, dist):
                "h2d_bytes_per_step": nb, "d2h_bytes_per_step": nb, "steps": e2e_steps,
                "api": "ps3d_gpu_advance_host (svor FP64 in/out)", "host_buffer": host_kind}
 
-    # FP64 form against the FP64 ALU roofline (flop model: 49 transforms per
-    # impl-diff-rk4 step at 2.5 N log2 n each, plus ~300 flop per point for
-    # the strain eigen-solve) and cuFFT as a comparator for the horizontal
-    # transforms
+    # FP64 form against the copy bandwidth: the fields that the stages of an
+    # impl-diff-rk4 step read and write, each once (1120 bytes per grid value;
+    # its transforms run on the integer pipes, so a count of FP64 operations
+    # has no peak to stand against); and cuFFT as a comparator for the
+    # horizontal transforms
     if fp64 is not None:
-        pk = fp64_peak_tflops(dev)
-        N = float(n) ** 2 * (n + 1)
-        flops = 49 * 2.5 * N * (3 * np.log2(n)) + 300.0 * N
-        ach = flops / (fp64["ms_per_step"] * 1e-3) / 1e12
-        fp64["alu"] = {"flops_per_step": flops, "achieved_tflops": ach, "peak_tflops": pk,
-                       "frac": (ach / pk) if pk else None,
-                       "peak_source": "cuBLAS DGEMM 4096^3 through torch, best of 5"}
+        nbytes = 1120.0 * float(n) ** 2 * (n + 1)
+        gbs = nbytes / (fp64["ms_per_step"] * 1e-3) / 1e9
+        fp64["hbm"] = {"bytes_per_step": nbytes, "achieved_gbs": gbs, "peak_gbs": peak, "frac": gbs / peak,
+                       "peak_source": peak_kind}
     cufft = None
     if rank == 0:
         cufft = cufft_comparator(n, dev)

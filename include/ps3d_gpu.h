@@ -174,7 +174,9 @@ int ps3d_gpu_vor2vel(ps3d_gpu_ctx *ctx);
  * part of the tendency's solenoidal projection, which its stage updates
  * use to project each source term as they apply it. */
 int ps3d_gpu_source(ps3d_gpu_ctx *ctx);
-/* adapt (advance.f90:109-377) incl. set_diffusion of the stepper */
+/* adapt (advance.f90:109-377) incl. set_diffusion of the stepper.  The FP64
+ * form runs the reference's Jacobi sweeps at the points that can hold a strain
+ * maximum, so a sweep limit (PS3D_ERR_DEVICE_LIMIT) is reported for those. */
 int ps3d_gpu_adapt(ps3d_gpu_ctx *ctx, double t, double *dt, ps3d_gpu_diag *diag);
 /* base_stepper%set_diffusion (impl_rk4.f90:37-53, cn2.f90:40-77) with the
  * vorticity prefactor (the buoyancy prefactor 0) */

@@ -1521,7 +1521,9 @@ __global__ void k_red1(Dims d, const T *__restrict__ vel, const T *__restrict__ 
 
 // The FP64 form of pass 1: the maxima compare bit patterns and only the end
 // levels are halved; every term enters its compensated accumulator.  The FP64
-// pipe bounds it (33 operations per element instead of about 50).
+// pipe bounds it (33 operations per element instead of about 50; 256^3: 2174 us
+// by the general kernel, 1382 here; 658 with a column's terms added plainly,
+// which loses the small ones).
 __device__ __forceinline__ long long order_key(double x)
 {
     const long long b = __double_as_longlong(x);
@@ -1732,7 +1734,10 @@ __global__ void k_red2(Dims d, const float *__restrict__ vor, const float *__res
 // largest one.  SCREEN is 30 times the estimate's error (the extreme
 // eigenvalues are a few FP32 units off, see sym3_maxabs), so the points that
 // hold the maxima are among them and the results are those of the full sweep.
-// An estimate that is not a number counts as within reach.
+// An estimate that is not a number counts as within reach.  The sweep limit is
+// raised by the points that are swept; no trace-free matrix that reaches it is
+// known (3.6e8 tried: exponents over the range of FP64, equal, nearly equal and
+// zero entries, mixed scales).
 constexpr float SCREEN = 3.0e-5f;
 struct StrainPoint {
     double a00, a01, a02, a11, a12, a22;
