@@ -1522,7 +1522,7 @@ __global__ void k_red1(Dims d, const T *__restrict__ vel, const T *__restrict__ 
 // The FP64 form of pass 1: the maxima compare bit patterns and only the end
 // levels are halved; every term enters its compensated accumulator.  The FP64
 // pipe bounds it (33 operations per element instead of about 50; 256^3: 2174 us
-// by the general kernel, 1382 here; 658 with a column's terms added plainly,
+// by the general kernel, 1218 here; 658 with a column's terms added plainly,
 // which loses the small ones).
 __device__ __forceinline__ long long order_key(double x)
 {
@@ -1549,7 +1549,9 @@ __global__ void k_red1<double>(Dims d, const double *__restrict__ vel, const dou
          col += (long long)gridDim.x * COLS_PER_BLOCK) {
         const long long o = col * d.P;
 #pragma unroll 2
-        for (int iz = threadIdx.x; iz <= d.nz; iz += 32) {
+        for (int c0 = 0; c0 <= d.nz; c0 += 32) {
+            const int iz = c0 + threadIdx.x;
+            if (iz > d.nz) continue;
             const long long i = o + iz;
             double x = vor[i], y = vor[N + i], z = vor[2 * N + i];
             const double u = vel[i], v = vel[N + i], w = vel[2 * N + i];
@@ -1558,13 +1560,14 @@ __global__ void k_red1<double>(Dims d, const double *__restrict__ vel, const dou
             raise(vmx[0], u);
             raise(vmx[1], v);
             raise(vmx[2], w);
-            if (iz == 0 || iz == d.nz) {
-                w2 *= 0.5;
-                u2 *= 0.5;
-                h *= 0.5;
-                x *= 0.5;
-                y *= 0.5;
-                z *= 0.5;
+            if (c0 == 0 || c0 + 32 > d.nz) {  // the same for the whole warp: no cost elsewhere
+                const double wt = iz == 0 || iz == d.nz ? 0.5 : 1.0;
+                w2 *= wt;
+                u2 *= wt;
+                h *= wt;
+                x *= wt;
+                y *= wt;
+                z *= wt;
             }
             s_w2.add(w2);
             s_u2.add(u2);
