@@ -1764,7 +1764,10 @@ int ps3d_closure_train(ps3d_closure *cl, int iters, double lr0, double lr1, unsi
         images(cl, cl->st, it + 1 == iters);  // the steps use the warp engine's images
         if ((it & 63) == 63) {
             rc = ccheck(cl, "train");
-            if (rc) return rc;
+            if (rc) {
+                images(cl, cl->st);  // no engine is left with the weights of before
+                return rc;
+            }
         }
     }
     if (cudaStreamSynchronize(cl->st) != cudaSuccess) return ccheck(cl, "train");
