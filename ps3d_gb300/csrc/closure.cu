@@ -273,8 +273,9 @@ __global__ void __launch_bounds__(CONV_THREADS, 4) k_conv(ConvArgs a)
 // the grid through a wall meets dZ fragments whose rows there are zero (a mask
 // per row).  The last warp multiplies by ones: the bias.  A block per tap and
 // chunk read the same rows 28 times, and index arithmetic and staging, not the
-// tensor pipe, took its time: 32 -> 32 channels at 64^3 219 us, 99 us here, where the warp-level
-// products (about 240 TFLOP/s at most on this chip) bound it.
+// tensor pipe, took its time: 32 -> 32 channels at 64^3 219 us, 100 us here,
+// where the warp-level products (about 240 TFLOP/s at most on this chip) bound
+// it.
 // Segments of 512 points are summed in the order of the four warps that took
 // one each there, so the sums are bitwise those.
 template <int CIN, int COUT> struct WG {
@@ -916,14 +917,13 @@ __device__ __forceinline__ void mbar_arrive(uint32_t a)
 // Warp 16 (one elected lane) is the producer and issuer: TMA copies of tile
 // k-1+nbuf into the shared buffer freed by the products of tile k-1 (two
 // buffers left the copies' latency exposed; three or four where they fit), and
-// the
-// 9 x CIN/16 tcgen05.mma of tile k into TMEM accumulator k%2 once the
+// the 9 x CIN/16 tcgen05.mma of tile k into TMEM accumulator k%2 once the
 // epilogue has released it.  Warps 0-15 are the epilogue, eight for the even
 // tiles and eight for the odd ones: they wait for the products of tile k, read
 // their lane quarter (warp % 4) and column half (warp / 4 % 2) of the three
-// accumulators, release them, exchange the rows next
-// to a quarter's edge through shared memory, and apply bias + GELU and the
-// stores.  The roles meet only on mbarriers: full[b] (copies landed), done[b]
+// accumulators, exchange the rows next to a quarter's edge through shared
+// memory, release the accumulators, and apply bias + GELU and the stores.
+// The roles meet only on mbarriers: full[b] (copies landed), done[b]
 // (products complete, tcgen05.commit), free[b] (256 epilogue arrivals), and
 // edge[b][half] (the four warps of a column half have put their edge rows).
 // Every wait is bounded; a wait that runs out sets a shared flag that stops
@@ -1109,7 +1109,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_conv_tc(TcArgs a)
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    if (warp == TC_ISSUER) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;\n" ::"r"(tmem) : "memory");
+    if (warp == TC_ISSUER)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 256;\n" ::"r"(tmem) : "memory");
 }
 
 // host-side SplitMix64 (parameter initialisation, sample order)
@@ -1361,7 +1362,7 @@ template <int CIN, int COUT> void wgrad(ps3d_closure *cl, cudaStream_t st, const
         act, dz, cl->wpart, cl->nx, cl->ny, cl->Z, cl->npts);
     const int n = NTAP * CREAL_IN[l] * CREAL_OUT[l] + CREAL_OUT[l];
     k_wgrad_reduce<<<(n + 31) / 32, 256, 0, st>>>(cl->wpart, cl->nchunk, CIN, COUT, CREAL_IN[l], CREAL_OUT[l],
-                                                    cl->g + woff(l));
+                                                  cl->g + woff(l));
 }
 
 // backward pass after forward + k_loss (dz4 holds dL/dout): all parameter
@@ -1558,8 +1559,8 @@ int ps3d_closure_create(int nx, int ny, int nz, int max_samples, int device, uns
     cl->QN = (long long)(nx + 2) * cl->YP * cl->ZP;
     cl->GUARD = (long long)cl->YP * cl->ZP + cl->ZP + 256;
     cl->RTOT = (cl->QN + 2 * cl->GUARD + 7) / 8 * 8;
-    cl->tc_ok = tc_smem<32, 32>(cl->ZP) + TC_STATIC <= (size_t)prop.sharedMemPerBlockOptin && tc_attr<16, 32, EPI_GELU>(cl) &&
-                tc_attr<32, 32, EPI_GELU>(cl) && tc_attr<32, 16, EPI_OUT>(cl);
+    cl->tc_ok = tc_smem<32, 32>(cl->ZP) + TC_STATIC <= (size_t)prop.sharedMemPerBlockOptin &&
+                tc_attr<16, 32, EPI_GELU>(cl) && tc_attr<32, 32, EPI_GELU>(cl) && tc_attr<32, 16, EPI_OUT>(cl);
     cl->engine = cl->tc_ok ? PS3D_CLOSURE_ENGINE_TCGEN05 : PS3D_CLOSURE_ENGINE_MMA;
     const long long P = cl->npts;
     bool ok = calloc_dev(cl, &cl->w, NPARAM * 4) && calloc_dev(cl, &cl->g, NPARAM * 4) &&

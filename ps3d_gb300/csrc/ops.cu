@@ -1731,9 +1731,9 @@ __global__ void k_red2(Dims d, const float *__restrict__ vor, const float *__res
 
 // The FP64 form takes the strain maxima from the reference's Jacobi sweeps,
 // but only the points that can hold a maximum need them (256^3: 22.7 ms on the
-// FP64 pipe when every point ran them, 0.71 ms with the screen).  k_red2_screen evaluates the closed form
-// in FP32 at every point and keeps its largest value per chunk of 32 levels;
-// k_strain_max runs the sweeps where the estimate comes within SCREEN of the
+// FP64 pipe when every point ran them, 0.71 ms with the screen).  k_red2_screen
+// evaluates the closed form in FP32 at every point and keeps its largest value
+// per chunk of 32 levels; k_strain_max runs the sweeps where the estimate comes within SCREEN of the
 // largest one.  SCREEN is 30 times the estimate's error (the extreme
 // eigenvalues are a few FP32 units off, see sym3_maxabs), so the points that
 // hold the maxima are among them and the results are those of the full sweep.
@@ -1828,7 +1828,8 @@ __global__ void k_strain_max(Dims d, const double *__restrict__ vor, const doubl
             bool want = false;
             if (c0 + lane < d.ncol) {
                 const float *e = est + (c0 + lane) * ep;
-                want = !(e[ch] < lim[0]) || (ch == d.nz >> 5 && !(e[nch] < lim[1])) || (ch == 0 && !(e[nch + 1] < lim[2]));
+                want = !(e[ch] < lim[0]) || (ch == d.nz >> 5 && !(e[nch] < lim[1])) ||
+                       (ch == 0 && !(e[nch + 1] < lim[2]));
             }
             for (unsigned todo = __ballot_sync(0xffffffffu, want); todo; todo &= todo - 1) {
                 const long long col = c0 + __ffs(todo) - 1;

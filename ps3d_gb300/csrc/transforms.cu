@@ -158,8 +158,8 @@ void y_forward(const Dims &d, cudaStream_t st, const T *in, T *out, const typena
                int nf)
 {
     if (pr) pr->begin(PROBE_YLINES, st);
-    launch_lines<T>(st, in, out, d.ny, d.P, d.nz + 1, d.P, d.nx, (long long)d.ny * d.P, false, twy, d.fx64, d.line_shape[0],
-                    nf, d.nfield, d.nfield);
+    launch_lines<T>(st, in, out, d.ny, d.P, d.nz + 1, d.P, d.nx, (long long)d.ny * d.P, false, twy, d.fx64,
+                    d.line_shape[0], nf, d.nfield, d.nfield);
     if (pr) pr->end(PROBE_YLINES, st, nf * pass_bytes<T>(d));
 }
 
@@ -168,8 +168,8 @@ void x_forward(const Dims &d, cudaStream_t st, const T *in, T *out, const typena
                int nf)
 {
     if (pr) pr->begin(PROBE_XLINES, st);
-    launch_lines<T>(st, in, out, d.nx, d.P, d.nz + 1, (long long)d.ny * d.P, d.ny, d.P, false, twx, d.fx64, d.line_shape[1],
-                    nf, d.nfield, d.nfield);
+    launch_lines<T>(st, in, out, d.nx, d.P, d.nz + 1, (long long)d.ny * d.P, d.ny, d.P, false, twx, d.fx64,
+                    d.line_shape[1], nf, d.nfield, d.nfield);
     if (pr) pr->end(PROBE_XLINES, st, nf * pass_bytes<T>(d));
 }
 
@@ -178,8 +178,8 @@ void x_inverse(const Dims &d, cudaStream_t st, const T *in, T *out, const typena
                int nf)
 {
     if (pr) pr->begin(PROBE_XLINES, st);
-    launch_lines<T>(st, in, out, d.nx, d.P, d.nz + 1, (long long)d.ny * d.P, d.ny, d.P, true, twx, d.fx64, d.line_shape[3],
-                    nf, d.nfield, d.nfield);
+    launch_lines<T>(st, in, out, d.nx, d.P, d.nz + 1, (long long)d.ny * d.P, d.ny, d.P, true, twx, d.fx64,
+                    d.line_shape[3], nf, d.nfield, d.nfield);
     if (pr) pr->end(PROBE_XLINES, st, nf * pass_bytes<T>(d));
 }
 
@@ -188,8 +188,8 @@ void y_inverse(const Dims &d, cudaStream_t st, const T *in, T *out, const typena
                int nf)
 {
     if (pr) pr->begin(PROBE_YLINES, st);
-    launch_lines<T>(st, in, out, d.ny, d.P, d.nz + 1, d.P, d.nx, (long long)d.ny * d.P, true, twy, d.fx64, d.line_shape[2],
-                    nf, d.nfield, d.nfield);
+    launch_lines<T>(st, in, out, d.ny, d.P, d.nz + 1, d.P, d.nx, (long long)d.ny * d.P, true, twy, d.fx64,
+                    d.line_shape[2], nf, d.nfield, d.nfield);
     if (pr) pr->end(PROBE_YLINES, st, nf * pass_bytes<T>(d));
 }
 
